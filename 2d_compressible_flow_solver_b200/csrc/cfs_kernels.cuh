@@ -136,6 +136,18 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
+// NaN-propagating minimum and maximum (one instruction each).
+__device__ __forceinline__ float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 template <class C> __device__ __forceinline__ C min_ref(C a, C b) { return (b < a) ? b : a; }
 template <class C> __device__ __forceinline__ C max_ref(C a, C b) { return (a < b) ? b : a; }
 
@@ -311,31 +323,33 @@ __device__ __forceinline__ void hll_flux(const Face5<typename Pol::C>& L, const 
             SR = fmax(uL + aL, uR + aR);
         }
     }
-    if constexpr (Pol::kMixed) {
-        // the HLL average on (rho, m_x) and (m_y, E) in packed FP32, then the
-        // upwind cases as selects
-        const float inv = rcp_fast(SR - SL);
-        const float2 sr = p2(SR), msl = p2(-SL), slsr = p2(SL * SR), iv = p2(inv);
-        const float2 H01 = mul2(fma2(slsr, sub2(make_float2(R.r, R.mx), make_float2(L.r, L.mx)),
-                                     fma2(msl, make_float2(FR[0], FR[1]), mul2(sr, make_float2(FL[0], FL[1])))), iv);
-        const float2 H23 = mul2(fma2(slsr, sub2(make_float2(R.my, R.E), make_float2(L.my, L.E)),
-                                     fma2(msl, make_float2(FR[2], FR[3]), mul2(sr, make_float2(FL[2], FL[3])))), iv);
-        const float H[4] = {H01.x, H01.y, H23.x, H23.y};
+    if constexpr (!Pol::kExact) {
+        // The HLL average written from the left flux, F = FL + w (SR dU - dF)
+        // with w = SL / (SR - SL), and the bounds clamped to SL <= 0 <= SR:
+        // where SL >= 0 the weight is 0 (F = FL exactly), where SR <= 0 it is
+        // -1 (F = FL + dF, the right flux to rounding), so no upwind selects
+        // remain.  A NaN bound stays NaN and gives a NaN flux, and the floor
+        // on SR keeps the reciprocal's argument positive.  Per face 8 packed
+        // instructions (FP32) and no selects, against 10 and 8 for the average
+        // formed from both fluxes and selected; 16 FP64 operations against 20.
+        if constexpr (Pol::kMixed) {
+            const float SLm = min_nan(SL, 0.0f), SRp = max_nan(SR, 1e-30f);
+            const float2 w = p2(SLm * rcp_fast(SRp - SLm)), sr = p2(SRp);
+            const float2 L01 = make_float2(FL[0], FL[1]), L23 = make_float2(FL[2], FL[3]);
+            const float2 F01 = fma2(w, fma2(sr, sub2(make_float2(R.r, R.mx), make_float2(L.r, L.mx)),
+                                            sub2(L01, make_float2(FR[0], FR[1]))), L01);
+            const float2 F23 = fma2(w, fma2(sr, sub2(make_float2(R.my, R.E), make_float2(L.my, L.E)),
+                                            sub2(L23, make_float2(FR[2], FR[3]))), L23);
+            F[0] = F01.x;
+            F[1] = F01.y;
+            F[2] = F23.x;
+            F[3] = F23.y;
+        } else {
+            const C SLm = SL >= 0 ? C(0) : SL, SRp = SR <= 0 ? C(1e-290) : SR;
+            const C w = SLm * rcp_pos(SRp - SLm);
+            const C dU[4] = {R.r - L.r, R.mx - L.mx, R.my - L.my, R.E - L.E};
 #pragma unroll
-        for (int q = 0; q < 4; ++q) F[q] = SL >= 0 ? FL[q] : (SR <= 0 ? FR[q] : H[q]);
-        return;
-    } else if constexpr (!Pol::kExact) {
-        // FP64 throughput form: the same shape (the average formed for every
-        // face, the upwind cases selected), so no divergent branch splits the
-        // face's arithmetic; where the average is selected SL < 0 < SR, so its
-        // reciprocal's argument is positive (elsewhere a NaN average is
-        // formed and not selected)
-        const C inv = rcp_pos(SR - SL), slsr = SL * SR;
-        const C dU[4] = {R.r - L.r, R.mx - L.mx, R.my - L.my, R.E - L.E};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const C H = fma(slsr, dU[q], fma(SR, FL[q], -SL * FR[q])) * inv;
-            F[q] = SL >= 0 ? FL[q] : (SR <= 0 ? FR[q] : H);
+            for (int q = 0; q < 4; ++q) F[q] = fma(w, fma(SRp, dU[q], FL[q] - FR[q]), FL[q]);
         }
         return;
     }
@@ -346,7 +360,7 @@ __device__ __forceinline__ void hll_flux(const Face5<typename Pol::C>& L, const 
 #pragma unroll
         for (int q = 0; q < 4; ++q) F[q] = FR[q];
     } else {
-        const C inv_SR_SL = Pol::kExact ? C(1.0) / (SR - SL) : rcp_fast(SR - SL);
+        const C inv_SR_SL = C(1.0) / (SR - SL);
         const C dU[4] = {R.r - L.r, R.mx - L.mx, R.my - L.my, R.E - L.E};
 #pragma unroll
         for (int q = 0; q < 4; ++q) F[q] = (SR * FL[q] - SL * FR[q] + SL * SR * dU[q]) * inv_SR_SL;

@@ -30,87 +30,89 @@ constexpr int kSeg = 30;
 // smoothness indicators and weight products and are formed as v2 plus a small
 // correction (fewer operations, and in FP32 a rounding error relative to the
 // correction instead of to the value):
-//   beta_k (13/12) d_k^2 + (1/4) e_k^2 with d = (D2-D1, D3-D2, D4-D3),
-//     e = (3 D2 - D1, D2 + D3, D4 - 3 D3) = (2 D2 + d0, D2 + D3, D4 - 3 D3);
-//     scaled by 12/13 with eps alike, which leaves the normalised weights
-//     unchanged;
-//   candidate p_k = v2 + c_k: c = ((5 D2 - 2 D1)/6, (D2 + 2 D3)/6, (4 D3 - D4)/6),
-//     mirrored c' = ((2 D4 - 5 D3)/6, -(D3 + 2 D2)/6, (D1 - 4 D2)/6); each
-//     mirrored candidate is d/6 minus a left one: c'_0 = d2/6 - c_2,
-//     c'_1 = d1/6 - c_1, c'_2 = d0/6 - c_0, so the left ones are formed
-//     negated (n_k = -c_k) and the right ones take one fused multiply-add;
-//   weights d_k / q_k with q_k = (eps + beta_k)^2, taken as products of the
-//     other two q times (1, 6, 3) (the linear weights 0.1, 0.6, 0.3 times 10).
+//   indicators: 13/12 d^2 + 1/4 e^2 with (d, e) = (D2-D1, 3 D2-D1),
+//     (D3-D2, D2+D3), (D4-D3, D4-3 D3), multiplied out and scaled by 3/4 (with
+//     eps alike, which leaves the normalised weights unchanged) so that every
+//     coefficient is a short binary fraction and eps enters a fused
+//     multiply-add:
+//       D1 (D1 - 11/4 D2) + 5/2 D2^2,  D2 (D2 - 5/4 D3) + D3^2,
+//       D4 (D4 - 11/4 D3) + 5/2 D3^2;
+//     the forms are positive definite (at least 0.24 D1^2, 0.61 D2^2, ...), so
+//     multiplying out costs a relative rounding of at most about 13 units in an
+//     indicator and no sign;
+//   weights d_k / q_k with q_k = (eps + beta_k)^2 as products of the other two
+//     q: X = q1 q2, Y = q0 q2, Z = q0 q1 times (1, 6, 3) on the left, (3, 6, 1)
+//     on the right (the linear weights 0.1, 0.6, 0.3 times 10);
+//   candidates v2 + c_k: c = (5/6 A0, A1/3, 2/3 A2) with A0 = D2 - 2/5 D1,
+//     A1 = D3 + 1/2 D2, A2 = D3 - 1/4 D4, one fused multiply-add each, and
+//     mirrored with a sign on the right (D1 <-> D4, D2 <-> D3);
+//   left  = v2 + (5/12 X A0 + Y A1 + Z A2) / (X/2 + 3 Y + 3/2 Z),
+//   right = v2 - (5/12 Z B0 + Y B1 + X B2) / (Z/2 + 3 Y + 3/2 X), the sums as
+//     3/2 (X + Z + 2 Y) - X and - Z.
+// 41 operations and two reciprocals per variable (52 before, with d, e and the
+// candidates formed separately): the row march is bound by issue (FP32) and
+// by the FP64 pipe, and this is more than half of its arithmetic.  Measured with
+// the HLL flux written from the left flux (hll_flux): SSP3 step of 4096^2
+// FP32-mixed 1,536 -> 1,412 us, of 2048^2 FP64 759 -> 690 us.
 template <class C>
 __device__ __forceinline__ void weno5_pair_diff(C v0, C v1, C v2, C v3, C v4, C eps, C& left, C& right) {
     const C D1 = v1 - v0, D2 = v2 - v1, D3 = v3 - v2, D4 = v4 - v3;
-    const C d0 = D2 - D1, d1 = D3 - D2, d2 = D4 - D3;
-    const C e0 = fma(C(2), D2, d0), e1 = D2 + D3, e2 = fma(C(-3), D3, D4);
-    const C k = C(3.0 / 13.0);
-    C b0 = fma(d0, d0, k * (e0 * e0));
-    C b1 = fma(d1, d1, k * (e1 * e1));
-    C b2 = fma(d2, d2, k * (e2 * e2));
+    const C P2 = D2 * D2, P3 = D3 * D3;
+    C q0 = fma(D1, fma(C(-2.75), D2, D1), fma(C(2.5), P2, eps));  // eps: the WENO eps times 3/4
+    C q1 = fma(D2, fma(C(-1.25), D3, D2), P3 + eps);
+    C q2 = fma(D4, fma(C(-2.75), D3, D4), fma(C(2.5), P3, eps));
     if (sizeof(C) == 4) {
-        b0 = fmin(b0, C(1e9));
-        b1 = fmin(b1, C(1e9));
-        b2 = fmin(b2, C(1e9));
+        q0 = fmin(q0, C(1e9));
+        q1 = fmin(q1, C(1e9));
+        q2 = fmin(q2, C(1e9));
     }
-    C q0 = eps + b0, q1 = eps + b1, q2 = eps + b2;  // eps: the WENO eps times 12/13
     q0 *= q0;
     q1 *= q1;
     q2 *= q2;
-    const C q01 = q0 * q1, q12 = q1 * q2, a1 = C(6) * (q0 * q2);
-    const C a2L = C(3) * q01, a2R = C(3) * q12;
-    const C n0 = fma(C(-5.0 / 6.0), D2, C(1.0 / 3.0) * D1);
-    const C n1 = fma(C(-1.0 / 3.0), D3, C(-1.0 / 6.0) * D2);
-    const C n2 = fma(C(-2.0 / 3.0), D3, C(1.0 / 6.0) * D4);
-    const C r0 = fma(C(1.0 / 6.0), d2, n2);
-    const C r1 = fma(C(1.0 / 6.0), d1, n1);
-    const C r2 = fma(C(1.0 / 6.0), d0, n0);
-    // (the weight sums are >= eps^2 > 0: rcp_pos; the left one negated after)
-    left = fma(fma(q12, n0, fma(a1, n1, a2L * n2)), -rcp_pos(q12 + a1 + a2L), v2);
-    right = fma(fma(q01, r0, fma(a1, r1, a2R * r2)), rcp_pos(q01 + a1 + a2R), v2);
+    const C X = q1 * q2, Y = q0 * q2, Z = q0 * q1;
+    const C X5 = C(5.0 / 12.0) * X, Z5 = C(5.0 / 12.0) * Z;
+    const C h = fma(C(2), Y, X + Z);
+    const C A0 = fma(C(-0.4), D1, D2), A1 = fma(C(0.5), D2, D3), A2 = fma(C(-0.25), D4, D3);
+    const C B0 = fma(C(-0.4), D4, D3), B1 = fma(C(0.5), D3, D2), B2 = fma(C(-0.25), D1, D2);
+    // (the weight sums are >= 5 eps^4 > 0: rcp_pos)
+    left = fma(fma(X5, A0, fma(Y, A1, Z * A2)), rcp_pos(fma(C(1.5), h, -X)), v2);
+    right = fma(fma(Z5, B0, fma(Y, B1, X * B2)), -rcp_pos(fma(C(1.5), h, -Z)), v2);
 }
 
 template <class C>
 __device__ __forceinline__ void weno5_pair(C v0, C v1, C v2, C v3, C v4, C eps, C& left, C& right) {
-    weno5_pair_diff(v0, v1, v2, v3, v4, C(12.0 / 13.0) * eps, left, right);
+    weno5_pair_diff(v0, v1, v2, v3, v4, C(0.75) * eps, left, right);
 }
 
 // The same pair for two variables at once in packed FP32 (sm_100 FFMA2 /
 // FADD2 / FMUL2: two independent FP32 operations per instruction, each rounded
 // as its scalar form), for the FP32-mixed form, whose row loop is bound by
-// instruction issue.  The reciprocals stay scalar.
+// instruction issue.  The reciprocals and the caps of the indicators, which
+// keep the products finite at any jump, stay scalar.
+
+__device__ __forceinline__ float2 cap2(float2 q) { return make_float2(fminf(q.x, 1e9f), fminf(q.y, 1e9f)); }
 
 __device__ __forceinline__ void weno5_pair_x2(float2 v0, float2 v1, float2 v2, float2 v3, float2 v4, float eps,
                                               float2& left, float2& right) {
     const float2 D1 = sub2(v1, v0), D2 = sub2(v2, v1), D3 = sub2(v3, v2), D4 = sub2(v4, v3);
-    const float2 d0 = sub2(D2, D1), d1 = sub2(D3, D2), d2 = sub2(D4, D3);
-    const float2 e0 = fma2(p2(2.0f), D2, d0), e1 = add2(D2, D3), e2 = fma2(p2(-3.0f), D3, D4);
-    const float2 k = p2(float(3.0 / 13.0));
-    float2 b0 = fma2(d0, d0, mul2(k, mul2(e0, e0)));
-    float2 b1 = fma2(d1, d1, mul2(k, mul2(e1, e1)));
-    float2 b2 = fma2(d2, d2, mul2(k, mul2(e2, e2)));
-    b0 = make_float2(fminf(b0.x, 1e9f), fminf(b0.y, 1e9f));
-    b1 = make_float2(fminf(b1.x, 1e9f), fminf(b1.y, 1e9f));
-    b2 = make_float2(fminf(b2.x, 1e9f), fminf(b2.y, 1e9f));
-    const float2 es = p2(float(12.0 / 13.0) * eps);
-    float2 q0 = add2(es, b0), q1 = add2(es, b1), q2 = add2(es, b2);
+    const float2 P2 = mul2(D2, D2), P3 = mul2(D3, D3);
+    const float2 es = p2(0.75f * eps);
+    float2 q0 = cap2(fma2(D1, fma2(p2(-2.75f), D2, D1), fma2(p2(2.5f), P2, es)));
+    float2 q1 = cap2(fma2(D2, fma2(p2(-1.25f), D3, D2), add2(P3, es)));
+    float2 q2 = cap2(fma2(D4, fma2(p2(-2.75f), D3, D4), fma2(p2(2.5f), P3, es)));
     q0 = mul2(q0, q0);
     q1 = mul2(q1, q1);
     q2 = mul2(q2, q2);
-    const float2 q01 = mul2(q0, q1), q12 = mul2(q1, q2), a1 = mul2(p2(6.0f), mul2(q0, q2));
-    const float2 a2L = mul2(p2(3.0f), q01), a2R = mul2(p2(3.0f), q12);
-    const float2 n0 = fma2(p2(float(-5.0 / 6.0)), D2, mul2(p2(float(1.0 / 3.0)), D1));
-    const float2 n1 = fma2(p2(float(-1.0 / 3.0)), D3, mul2(p2(float(-1.0 / 6.0)), D2));
-    const float2 n2 = fma2(p2(float(-2.0 / 3.0)), D3, mul2(p2(float(1.0 / 6.0)), D4));
-    const float2 sixth = p2(float(1.0 / 6.0));
-    const float2 r0 = fma2(sixth, d2, n2), r1 = fma2(sixth, d1, n1), r2 = fma2(sixth, d0, n0);
-    const float2 sL = add2(add2(q12, a1), a2L), sR = add2(add2(q01, a1), a2R);
-    // (the left reciprocals negated: the left sum is over the negated candidates)
+    const float2 X = mul2(q1, q2), Y = mul2(q0, q2), Z = mul2(q0, q1);
+    const float2 X5 = mul2(p2(float(5.0 / 12.0)), X), Z5 = mul2(p2(float(5.0 / 12.0)), Z);
+    const float2 h = fma2(p2(2.0f), Y, add2(X, Z));
+    const float2 A0 = fma2(p2(-0.4f), D1, D2), A1 = fma2(p2(0.5f), D2, D3), A2 = fma2(p2(-0.25f), D4, D3);
+    const float2 B0 = fma2(p2(-0.4f), D4, D3), B1 = fma2(p2(0.5f), D3, D2), B2 = fma2(p2(-0.25f), D1, D2);
+    // (both sums negated, one packed operation each; the left reciprocals' sign is taken back in their argument)
+    const float2 sL = fma2(p2(-1.5f), h, X), sR = fma2(p2(-1.5f), h, Z);
     const float2 iL = make_float2(rcp_fast(-sL.x), rcp_fast(-sL.y)), iR = make_float2(rcp_fast(sR.x), rcp_fast(sR.y));
-    left = fma2(fma2(q12, n0, fma2(a1, n1, mul2(a2L, n2))), iL, v2);
-    right = fma2(fma2(q01, r0, fma2(a1, r1, mul2(a2R, r2))), iR, v2);
+    left = fma2(fma2(X5, A0, fma2(Y, A1, mul2(Z, A2))), iL, v2);
+    right = fma2(fma2(Z5, B0, fma2(Y, B1, mul2(X, B2))), iR, v2);
 }
 
 // finish_state of a cell's two states at once (FP32-mixed: packed
