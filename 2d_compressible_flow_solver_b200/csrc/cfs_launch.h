@@ -81,6 +81,37 @@ constexpr int kEdgeVariantF32 = 8;
 constexpr int kRingBlocksPerSmF64 = 4;
 constexpr int kWindowVariantF64 = 4;
 
+// Row chunk of a launch whose warps (nseg per chunk of rows, w per block) run
+// on `slots` resident blocks.  An item costs its R rows plus about 2 more (the x-work of
+// the row above and below the chunk), and the launch ends with a partly
+// filled stretch of about half an item, so the launch lasts about
+// (R + 2) (blocks / slots + 1/2): short chunks pay the per-item rows, long
+// ones the tail -- and, on a grid of few items, the chain of one warp's rows
+// (1.2 us a row in FP32, 2.0 in FP64), which is all that such a launch waits
+// for.  The minimum lies near R = 2 sqrt(nseg nrows / (w slots)): 28 rows
+// at 4096^2, 14 at 2048^2, 7 at 1024^2 (FP32, 740 slots), 2 at 256^2, 1 at
+// 64 x 48.  Fitted to a sweep of fixed chunks of 8 .. 196 rows at 512^2 ..
+// 4096^2, FP32 and FP64 (a whole-wave model that ignored the tail picked 196
+// rows at 4096^2 and lost 12 % against 32), and followed by a sweep of 1 .. 24
+// rows below: periodic SSP3 steps with chunks of at least 6 rows (the search's
+// end before) against the chosen ones, 64 x 48 FP64 49.2 -> 20.4 us, 256^2
+// FP32 37.0 -> 25.2, 512^2 FP32 51.2 -> 47.0.  Searched over 1 .. 128 rows
+// (the whole range when it is shorter), ties to the longer chunk.
+inline int choose_rows(int nseg, int w, int nrows, long long slots) {
+    int best_r = 32;
+    long long best_cost = -1;
+    const int r_max = nrows < 128 ? nrows : 128;
+    for (int r = 1; r <= r_max; ++r) {
+        const long long blocks = (static_cast<long long>(nseg) * ((nrows + r - 1) / r) + w - 1) / w;
+        const long long cost = static_cast<long long>(r + 2) * (2 * blocks + slots);
+        if (best_cost < 0 || cost <= best_cost) {
+            best_cost = cost;
+            best_r = r;
+        }
+    }
+    return best_r;
+}
+
 // Batched forms (cfs_batch_*): one launch covers every case of a batch.
 constexpr int kBatchWarps = 4;
 // 4 blocks of 4 warps per SM (128 registers): the uneven 512-case batch ran

@@ -2,7 +2,6 @@
 //   -DCFS_MARCH_POL=PolF32|PolF64  -DCFS_MARCH_FEAT=0..7  -DCFS_MARCH_FN=<launcher name>
 // (the build gives each pair its own object, so the 160 kernels compile in
 // parallel).  The launcher runs the variant `v` of kVariants (1-based).
-#include <climits>
 #include <mutex>
 
 #include "cfs_kernels.cuh"
@@ -17,33 +16,6 @@ namespace cfs {
 namespace {
 
 constexpr int kMaxDev = 64;
-
-// Row chunk of a launch whose warps (nseg per chunk of rows, w per block) run
-// on `slots` resident blocks.  An item costs its R rows plus about 2 more (the x-work of
-// the row above and below the chunk), and the launch ends with a partly
-// filled stretch of about half an item, so the launch lasts about
-// (R + 2) (blocks / slots + 1/2): short chunks pay the per-item rows, long
-// ones the tail.  The minimum lies near R = 2 sqrt(nseg nrows / (w slots)): 28 rows
-// at 4096^2, 14 at 2048^2, 7 at 1024^2 (FP32, 740 slots).  Fitted to a sweep of
-// fixed chunks of 8 .. 196 rows at 512^2 .. 4096^2, FP32 and FP64; a
-// whole-wave model that ignored the tail picked 196 rows at 4096^2 and lost
-// 12 % against 32.  Searched over 6 .. 128 rows (the whole range when it is
-// shorter), ties to the longer chunk.
-int choose_rows(int nseg, int w, int nrows, long long slots) {
-    if (nrows <= 6 || slots <= 0) return nrows <= 6 ? nrows : 32;
-    int best_r = 32;
-    long long best_cost = LLONG_MAX;
-    const int r_max = nrows < 128 ? nrows : 128;
-    for (int r = 6; r <= r_max; ++r) {
-        const long long blocks = (static_cast<long long>(nseg) * ((nrows + r - 1) / r) + w - 1) / w;
-        const long long cost = static_cast<long long>(r + 2) * (2 * blocks + slots);
-        if (cost <= best_cost) {
-            best_cost = cost;
-            best_r = r;
-        }
-    }
-    return best_r;
-}
 
 template <class Pol, int R, int W, int B, int Ld, int F>
 cudaError_t launch_march(const StageArgs& a_in, cudaStream_t s) {
