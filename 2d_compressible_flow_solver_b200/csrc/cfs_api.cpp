@@ -39,7 +39,7 @@ struct cfs_ctx {
     uint8_t* types_d = nullptr;
     uint8_t* lowo_d = nullptr;  // [nx+1][ny+1] face flags of CFS_POSITIVITY_BODY
     uint8_t* cflags_d = nullptr;  // [nx+2][ny+2] per-cell flags of the row march (with cell types)
-    void* bflux = nullptr;        // boundary-face fluxes of the row march (physical sides)
+    void* bflux = nullptr;        // boundary-face fluxes of the row march (Dirichlet sides)
     bool has_tmaps = false;       // throughput forms: TMA tensor maps of S0, S1, S2 encoded
     alignas(64) unsigned char tmaps[3][cfs::kTensorMapBytes] = {};
     unsigned int* err_d = nullptr;   // device error flags (cfs::kErr* bits)
@@ -485,9 +485,7 @@ int cfs_create(const cfs_config* cfg, cfs_ctx** out) {
         if (cudaMalloc(&c->rv, vb) != cudaSuccess) { c->err = "device allocation of the viscous RHS failed"; return bail(CFS_ERR_NOMEM); }
         cudaMemsetAsync(c->rv, 0, vb, c->stream);
     }
-    bool physical = false;
-    for (int s = 0; s < 4; ++s) physical = physical || cfg->bc[s] == CFS_BC_NEUMANN || cfg->bc[s] == CFS_BC_DIRICHLET;
-    if (physical && c->prec != cfs::kF64Exact) {
+    if (cfs::dirichlet_side(cfg->bc) && c->prec != cfs::kF64Exact) {
         const size_t bb = static_cast<size_t>(cfs::bflux_count(c->L)) * c->L.elem_bytes;
         if (cudaMalloc(&c->bflux, bb) != cudaSuccess) { c->err = "device allocation of the boundary fluxes failed"; return bail(CFS_ERR_NOMEM); }
     }

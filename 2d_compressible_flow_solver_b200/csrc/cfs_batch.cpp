@@ -61,7 +61,7 @@ struct cfs_batch {
     uint8_t* types_d = nullptr;
     uint8_t* lowo_d = nullptr;
     uint8_t* cflags_d = nullptr;
-    bool any_bflux = false;  // some case has a physical side
+    bool any_bflux = false;  // some case has a Dirichlet side
     std::vector<FeatureGroup> groups;  // work items by feature set, largest cases first in each
     int max_edge = 0;        // largest nx or ny of the cases
     int total_ig = 0;
@@ -320,9 +320,7 @@ int cfs_batch_create(const cfs_config* common, int ncases, const cfs_case* cases
         c.state_off = arena;
         arena += static_cast<size_t>(3) * static_cast<size_t>(c.L.bytes());
         arena = (arena + 255) & ~static_cast<size_t>(255);
-        bool physical = false;
-        for (int s = 0; s < 4; ++s) physical = physical || d.bc[s] == CFS_BC_NEUMANN || d.bc[s] == CFS_BC_DIRICHLET;
-        if (physical) {
+        if (cfs::dirichlet_side(d.bc)) {
             c.bflux_off = static_cast<long long>(arena);
             arena += static_cast<size_t>(cfs::bflux_count(c.L)) * b->elem;
             arena = (arena + 255) & ~static_cast<size_t>(255);

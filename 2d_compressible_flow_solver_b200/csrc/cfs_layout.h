@@ -104,7 +104,7 @@ struct StageArgs {
     unsigned int seed;     // stochastic-rounding step counter when P is null
     const uint8_t* cflags; // throughput forms: per-cell flag bytes (kCell* bits) of cells
                            // i = -1..nx, j = -1..ny, [nx+2][ny+2]; null = all fluid, no low-order faces
-    void* bflux;           // throughput forms: fluxes through the physical boundary faces
+    void* bflux;           // throughput forms: fluxes through the Dirichlet boundary faces
                            // (bflux_side_offset), arithmetic type of the form
     int row_lo, row_hi;    // throughput forms: the launch updates cells of rows [row_lo, row_hi)
                            // (row_hi 0: up to nx); a decomposed grid updates its interior
@@ -147,10 +147,16 @@ CFS_HD long long bflux_count(const Layout& L) { return 8LL * (L.nx + L.ny); }
 // Sides whose faces take the reference's boundary stencil.
 CFS_HD bool physical_side(const StageArgs& a, int s) { return a.bc[s] == kNeumann || a.bc[s] == kDirichlet; }
 
+// Whether some side takes its face fluxes from StageArgs::bflux (Dirichlet; a
+// transmissive face's flux is formed by the march).
+CFS_HD bool dirichlet_side(const int bc[4]) {
+    return bc[0] == kDirichlet || bc[1] == kDirichlet || bc[2] == kDirichlet || bc[3] == kDirichlet;
+}
+
 // Row-march instantiation features, chosen per launch:
 constexpr int kFeatPos = 1;    // positivity fallbacks and floors (StageArgs::positivity != 0)
 constexpr int kFeatExtra = 2;  // RHS copy (StageArgs::rhs) and viscous RHS (StageArgs::rv)
-constexpr int kFeatEdge = 4;   // physical sides (boundary-face fluxes) or cell flags (StageArgs::cflags)
+constexpr int kFeatEdge = 4;   // physical sides or cell flags (StageArgs::cflags)
 CFS_HD int march_features(const StageArgs& a) {
     bool edge = a.cflags != nullptr;
     for (int s = 0; s < 4; ++s) edge = edge || physical_side(a, s);

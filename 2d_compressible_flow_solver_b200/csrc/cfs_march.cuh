@@ -370,11 +370,33 @@ __device__ __forceinline__ void fix_face(bool low, const typename Pol::C cl[kVar
     fix_states<Pol>(false, low, cr, g, dummy, R);
 }
 
-// Fluxes through the physical boundary faces of one stage (the reference's
+// Flux through a transmissive face whose cell value is c: the ghosts repeat c
+// (NeummanBoundary.cpp:31-45), so the face's whole stencil [c c c | c c c]
+// reconstructs c on both sides (a positivity fallback gives c again) and the
+// HLL flux of two equal states is the physical flux; a negative pressure or
+// density (a NaN sound speed) still gives a NaN flux.
+template <class Pol>
+__device__ __forceinline__ void wall_flux(const typename Pol::C c[kVars], int dir, double g, typename Pol::C F[kVars]) {
+    using C = typename Pol::C;
+    Face5<C> s;
+    s.r = c[0];
+    s.mx = c[1];
+    s.my = c[2];
+    s.E = c[3];
+    finish_state<Pol>(s, g);
+    phys_flux<Pol>(s, dir, F);
+    const C nan_or_0 = s.a - s.a;
+#pragma unroll
+    for (int v = 0; v < kVars; ++v) F[v] += nan_or_0;
+}
+
+// Fluxes through the Dirichlet boundary faces of one stage (the reference's
 // boundary stencil [g g g | c c c], CellInterface.cpp:172-178, then the
 // positivity fallback and HLL), computed by boundary_flux_kernel before the
 // row march, which reads them (StageArgs::bflux) instead of reconstructing
-// there.
+// there.  (Transmissive faces need no stencil: the march forms them itself,
+// wall_flux, which saves their grids this launch -- 3.8 us a stage at
+// 64 x 48.)
 template <class Pol>
 __device__ __forceinline__ void boundary_face_flux(const StageArgs& a, int s, int k) {
     using T = typename Pol::T;
@@ -427,7 +449,7 @@ template <class Pol>
 __global__ void __launch_bounds__(128) boundary_flux_kernel(const StageArgs a) {
     const int s = blockIdx.y;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (!physical_side(a, s) || k >= (s < 2 ? a.L.ny : a.L.nx)) return;
+    if (a.bc[s] != kDirichlet || k >= (s < 2 ? a.L.ny : a.L.nx)) return;
     boundary_face_flux<Pol>(a, s, k);
 }
 
@@ -437,7 +459,7 @@ __global__ void __launch_bounds__(128) batch_boundary_flux_kernel(const StageArg
     const StageArgs& a = args[blockIdx.z];
     const int s = blockIdx.y;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (!a.bflux || !physical_side(a, s) || k >= (s < 2 ? a.L.ny : a.L.nx)) return;
+    if (!a.bflux || a.bc[s] != kDirichlet || k >= (s < 2 ? a.L.ny : a.L.nx)) return;
     boundary_face_flux<Pol>(a, s, k);
 }
 
@@ -459,8 +481,9 @@ __global__ void __launch_bounds__(128) batch_boundary_flux_kernel(const StageArg
 //     arithmetic (the FP64 form loads U^0 early in the row's iteration and
 //     keeps its ring in dynamic shared memory).
 //
-// The row loop holds no rarely taken code of any size: physical boundary faces
-// read the fluxes of boundary_flux_kernel and cell types and low-order faces
+// The row loop holds no rarely taken code of any size: a transmissive face's
+// flux is the cell's own (wall_flux), a Dirichlet one is read from
+// boundary_flux_kernel, and cell types and low-order faces
 // come from one flag byte per cell (StageArgs::cflags), both compiled in only
 // with kFeatEdge; the positivity fallback is a select of the cell's own state
 // (kFeatPos); the RHS copy and viscous RHS come with kFeatExtra.  A loop body that outgrows the
@@ -520,7 +543,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
     const bool last_of_step = a.rk == kRkTvd2 ? a.stage == 1 : a.stage == 2;
     const bool sr = Pol::kMixed && ((a.rounding == 0 && last_of_step) || a.rounding == 2);
     const unsigned int step_seed = (a.P ? a.P->seed[a.parity] : a.seed) * 4u + static_cast<unsigned int>(a.stage);
-    // physical boundary faces: fluxes precomputed (boundary_flux_kernel)
+    // physical boundary faces: the cell's own flux (transmissive) or a precomputed one (Dirichlet)
     const bool lo_x = kEdge && physical_side(a, 0), hi_x = kEdge && physical_side(a, 1);
     const bool lo_y = kEdge && physical_side(a, 2), hi_y = kEdge && physical_side(a, 3);
     const C* const bfl = static_cast<const C*>(a.bflux);
@@ -571,11 +594,11 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
         }
         return f;
     };
-    // this lane reconstructs the ghost column of a physical y side (its y-face
-    // flux is the boundary flux); warp-uniform screen for the rare lanes
+    // this lane's upper y-face is a physical one; warp-uniform screen for the rare lanes
     const bool ybnd = (j == -1 && lo_y) || (j == L.ny - 1 && hi_y);
     const bool warp_ybnd = __any_sync(0xffffffffu, ybnd);
-    const C* const bfy = ybnd ? bfl + bflux_side_offset(L, j == -1 ? 2 : 3) : nullptr;
+    const C* const bfy = ybnd && (j == -1 ? a.bc[2] == kDirichlet : a.bc[3] == kDirichlet)
+                             ? bfl + (j == -1 ? bflux_side_offset(L, 2) : bflux_side_offset(L, 3)) : nullptr;
     // RK operands of cell (i, j): the stored value (FP32 form), U^0.
     // (U^1, read by the reference's TVD3 stage 2 only, is loaded at its use.)
     T pf_cur[kVars], pf_u0[kVars];
@@ -742,8 +765,14 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
             // branch of its own would not overlap the surrounding work)
             hll_flux<Pol>(Lx, Rr, 0, a.hll, g, FX);
             if ((r == 0 && lo_x) || (r == L.nx && hi_x)) {  // uniform per warp
-                const C* b = bfl + bflux_side_offset(L, r == 0 ? 0 : 1);
-                if (j >= 0 && j < L.ny) {
+                // (no side index computed at run time: it would put the batch's argument block into local memory)
+                if (r == 0 ? a.bc[0] == kNeumann : a.bc[1] == kNeumann) {
+                    C c[kVars];
+                    if (r == 0) full(win[2], c);
+                    else full(win[1], c);
+                    wall_flux<Pol>(c, 0, g, FX);
+                } else if (j >= 0 && j < L.ny) {
+                    const C* b = bfl + bflux_side_offset(L, r == 0 ? 0 : 1);
 #pragma unroll
                     for (int v = 0; v < kVars; ++v) FX[v] = b[static_cast<long long>(v) * L.ny + j];
                 }
@@ -894,8 +923,16 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
             C FY[kVars];
             hll_flux<Pol>(Ly, Rn, 1, a.hll, g, FY);
             if (warp_ybnd && ybnd) {
+                if (bfy) {
 #pragma unroll
-                for (int v = 0; v < kVars; ++v) FY[v] = bfy[static_cast<long long>(v) * L.nx + r];
+                    for (int v = 0; v < kVars; ++v) FY[v] = bfy[static_cast<long long>(v) * L.nx + r];
+                } else {  // the interior cell: column 0 for the lane below it, this lane's at the top
+                    C c[kVars];
+#pragma unroll
+                    for (int v = 0; v < kVars; ++v) c[v] = j == -1 ? st[3][v] : st[2][v];
+                    full(c, c);
+                    wall_flux<Pol>(c, 1, g, FY);
+                }
             }
 #pragma unroll
             for (int v = 0; v < kVars; ++v) {

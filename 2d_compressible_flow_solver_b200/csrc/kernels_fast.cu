@@ -8,12 +8,11 @@
 
 namespace cfs {
 
-// Boundary-face fluxes of the stage (physical sides only), then the row march
+// Boundary-face fluxes of the stage (Dirichlet sides only), then the row march
 // of the stage's feature set.
 template <class Pol>
 cudaError_t launch_boundary_flux(const StageArgs& a, cudaStream_t s) {
-    if (!(physical_side(a, 0) || physical_side(a, 1) || physical_side(a, 2) || physical_side(a, 3)))
-        return cudaSuccess;
+    if (!dirichlet_side(a.bc)) return cudaSuccess;
     if (!a.bflux) return cudaErrorInvalidValue;
     const int n = a.L.nx > a.L.ny ? a.L.nx : a.L.ny;
     boundary_flux_kernel<Pol><<<dim3((n + 127) / 128, 4), 128, 0, s>>>(a);
@@ -151,7 +150,7 @@ cudaError_t launch_batch_stage(Prec p, const StageArgs* args, const int* item_ca
                                                                          case_nseg, total, counter, grid, feat, s);
 }
 
-// Boundary-face fluxes of every case of a batch (cases without physical sides
+// Boundary-face fluxes of every case of a batch (cases without Dirichlet sides
 // carry no bflux and return at once).
 cudaError_t launch_batch_boundary_flux(Prec p, const StageArgs* args, int ncases, int max_edge, cudaStream_t s) {
     for (int c0 = 0; c0 < ncases; c0 += 65535) {  // gridDim.z limit
