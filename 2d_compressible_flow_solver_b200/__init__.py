@@ -495,9 +495,15 @@ class Solver:
 class Batch:
     """Many independent grids advanced together (a ``cfs_batch``): one
     persistent launch per stage for all cases, per-case CFL dt on the device.
-    A case without ``rows`` takes the work-unit rows the autotuner measured
-    best for its size (``tuning.json`` ``batch_rows``; ``tuned_rows=False``:
-    the library default)."""
+    A case without ``rows`` takes, in a batch as large as the one they were
+    tuned on, the work-unit rows the autotuner measured best for its size
+    (``tuning.json`` ``batch_rows``), else the library's default, which follows
+    the batch's size (``tuned_rows=False``: always the default)."""
+
+    # cells from which the tuned rows (64 in every bucket, measured at 91 M
+    # cells) and the library's rule give the same estimated time; below, the
+    # tuned units are too long to fill the GPU
+    _TUNED_ROWS_MIN_CELLS = 32_000_000
 
     def __init__(self, cases, *, precision: int = FP32_MIXED, rk: int = RK_SSP3, hll: int = HLL_DAVIS,
                  gamma: float = 1.4, weno_eps: float = 1e-2, device: int = 0, positivity: int = POSITIVITY_OFF,
@@ -510,6 +516,7 @@ class Batch:
             int(precision), int(rk), int(hll), float(gamma), float(weno_eps), int(device))
         cfg.positivity, cfg.rounding = int(positivity), int(rounding)
         arr = (CfsCase * len(cases))()
+        tuned_rows = tuned_rows and sum(int(c["nx"]) * int(c["ny"]) for c in cases) >= self._TUNED_ROWS_MIN_CELLS
         self.shapes = []
         for k, c in enumerate(cases):
             d = arr[k]

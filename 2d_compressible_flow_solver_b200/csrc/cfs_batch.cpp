@@ -46,7 +46,6 @@ struct FeatureGroup {
     int feat = 0;
     int first = 0, count = 0;  // range of the group's items in item_case / item_local
 };
-constexpr int kMaxGroups = 4;  // the feature sets a batch launches: 0, Pos, Edge, Edge | Pos
 
 }  // namespace
 
@@ -80,7 +79,7 @@ struct cfs_batch {
     int* item_local = nullptr;
     int* case_rows = nullptr;
     int* case_nseg = nullptr;
-    unsigned int* counters = nullptr;  // [parity][stage][group]
+    unsigned int* counters = nullptr;  // [parity][stage][group] (cfs::kBatchCounters)
     double* staging = nullptr;
     double* sums = nullptr;  // plane sums of an uploaded case state (FP32 storage offsets)
     int grid = 0;
@@ -117,6 +116,31 @@ int stages_of(int rk) { return rk == CFS_RK_TVD2 ? 2 : 3; }
 
 // FP64 bit pattern of +infinity: the CFL maximum of a state with a non-finite fluid cell
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
+
+// Rows of a work unit where a case sets none: the chunk of the single-grid
+// launches (choose_rows), over the units of all cases and the `warps` resident
+// ones -- a unit of R rows costs about R + 2, and a stage lasts about
+// (R + 2) (units / warps + 1/2).  A large batch gets long units (71 rows on
+// 512 uneven cases of 64 .. 768 cells, where a sweep had found 64 to 96 best),
+// a small one short ones, or most warps would find no unit.  SSP3 steps with
+// 64 rows (the default before) and these, FP32 / FP64: 4 cases to 256 cells
+// 440 -> 66 / 694 -> 93 us, 24 to 512 562 -> 306 / 949 -> 491, 48 to 768
+// 1,123 -> 1,020 / 1,917 -> 1,697; within 2 % of the best of a sweep of 2 ..
+// 96 rows from 8 to 256 cases.
+int default_rows(const std::vector<BatchCase>& cases, long long warps) {
+    int best_r = cfs::kBatchMaxRows;
+    long long best_cost = -1;
+    for (int r = 1; r <= cfs::kBatchMaxRows; ++r) {
+        long long units = 0;
+        for (const BatchCase& c : cases) units += static_cast<long long>(c.nseg) * ((c.desc.nx + r - 1) / r);
+        const long long cost = static_cast<long long>(r + 2) * (2 * units + warps);
+        if (best_cost < 0 || cost <= best_cost) {
+            best_cost = cost;
+            best_r = r;
+        }
+    }
+    return best_r;
+}
 
 void* state_buf(const cfs_batch* b, const BatchCase& c, int k) {
     return b->arena + c.state_off + static_cast<size_t>(k) * static_cast<size_t>(c.L.bytes());
@@ -198,7 +222,6 @@ int enqueue_batch_step(cfs_batch* b, int parity) {
     for (int s = 0; s < S; ++s) {
         const int slot = parity * 3 + s;
         const int in = s;  // stage s reads S_s (S0, S1, S2)
-        CFSB_CUDA(b, cudaMemsetAsync(b->counters + slot * kMaxGroups, 0, sizeof(unsigned int) * kMaxGroups, b->stream));
         if (b->total_ig > 0)
             CFSB_CUDA(b, cfs::launch_batch_ib_fill(b->elem, b->dib + static_cast<size_t>(in) * b->n, b->ig_case,
                                                    b->ig_local, b->total_ig, b->stream));
@@ -209,8 +232,8 @@ int enqueue_batch_step(cfs_batch* b, int parity) {
             const FeatureGroup& fg = b->groups[g];
             CFSB_CUDA(b, cfs::launch_batch_stage(b->prec, b->dargs + static_cast<size_t>(slot) * b->n,
                                                  b->item_case + fg.first, b->item_local + fg.first, b->case_rows,
-                                                 b->case_nseg, fg.count, b->counters + slot * kMaxGroups + g, b->grid,
-                                                 fg.feat, b->stream));
+                                                 b->case_nseg, fg.count, b->counters, slot * cfs::kBatchMaxGroups + static_cast<int>(g),
+                                                 b->grid, fg.feat, b->stream));
         }
     }
     return CFS_OK;
@@ -314,9 +337,7 @@ int cfs_batch_create(const cfs_config* common, int ncases, const cfs_case* cases
         c.L = cfs::Layout::make(d.nx, d.ny, b->elem);
         c.dx = d.lx / d.nx;
         c.dy = d.ly / d.ny;
-        c.rows = d.rows > 0 ? d.rows : cfs::kBatchRows;
         c.nseg = (d.ny + 29) / 30;
-        c.items_y = (d.nx + c.rows - 1) / c.rows;
         c.state_off = arena;
         arena += static_cast<size_t>(3) * static_cast<size_t>(c.L.bytes());
         arena = (arena + 255) & ~static_cast<size_t>(255);
@@ -368,6 +389,17 @@ int cfs_batch_create(const cfs_config* common, int ncases, const cfs_case* cases
         }
     }
     b->total_ig = static_cast<int>(h_cell.size());
+
+    // --- rows of a work unit, for the cases that leave them to the library
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, common->device) != cudaSuccess || sms <= 0)
+        return bail(CFS_ERR_CUDA, "SM count query failed");
+    b->grid = sms * cfs::batch_blocks_per_sm(b->prec);
+    const int rows = default_rows(b->cases, static_cast<long long>(b->grid) * cfs::kBatchWarps);
+    for (BatchCase& c : b->cases) {
+        c.rows = c.desc.rows > 0 ? c.desc.rows : rows;
+        c.items_y = (c.desc.nx + c.rows - 1) / c.rows;
+    }
 
     // --- features per case: edge code where a case has a physical side or
     // a body, positivity code as the batch's mode asks
@@ -428,7 +460,7 @@ int cfs_batch_create(const cfs_config* common, int ncases, const cfs_case* cases
         !dalloc(reinterpret_cast<void**>(&b->item_local), sizeof(int) * it_local.size()) ||
         !dalloc(reinterpret_cast<void**>(&b->case_rows), sizeof(int) * ncases) ||
         !dalloc(reinterpret_cast<void**>(&b->case_nseg), sizeof(int) * ncases) ||
-        !dalloc(reinterpret_cast<void**>(&b->counters), sizeof(unsigned int) * 6 * kMaxGroups) ||
+        !dalloc(reinterpret_cast<void**>(&b->counters), sizeof(unsigned int) * cfs::kBatchCounters) ||
         !dalloc(reinterpret_cast<void**>(&b->staging), sizeof(double) * kVars * max_cells) ||
         !dalloc(reinterpret_cast<void**>(&b->sums), sizeof(double) * cfs::plane_sums_scratch_doubles()))
         return bail(CFS_ERR_NOMEM, "batch device allocation failed");
@@ -452,6 +484,7 @@ int cfs_batch_create(const cfs_config* common, int ncases, const cfs_case* cases
          h2d(b->item_case, it_case.data(), sizeof(int) * it_case.size()) &&
          h2d(b->item_local, it_local.data(), sizeof(int) * it_local.size()) &&
          h2d(b->case_rows, c_rows.data(), sizeof(int) * ncases) && h2d(b->case_nseg, c_ix.data(), sizeof(int) * ncases) &&
+         cudaMemset(b->counters, 0, sizeof(unsigned int) * cfs::kBatchCounters) == cudaSuccess &&
          cudaMemset(b->P, 0, sizeof(cfs::DevParams) * ncases) == cudaSuccess;
     if (!ok) return bail(CFS_ERR_CUDA, "batch upload failed");
     for (int ci = 0; ci < ncases; ++ci)
@@ -459,10 +492,6 @@ int cfs_batch_create(const cfs_config* common, int ncases, const cfs_case* cases
             if (cfs::launch_ghost_fill(b->elem, state_buf(b, b->cases[ci], k), b->cases[ci].L, b->cases[ci].sides,
                                        b->stream) != cudaSuccess)
                 return bail(CFS_ERR_CUDA, "ghost fill failed");
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, common->device) != cudaSuccess || sms <= 0)
-        return bail(CFS_ERR_CUDA, "SM count query failed");
-    b->grid = sms * cfs::batch_blocks_per_sm(b->prec);
     if (cudaStreamSynchronize(b->stream) != cudaSuccess || cudaGetLastError() != cudaSuccess)
         return bail(CFS_ERR_CUDA, "batch initialisation failed");
     *out = b;
@@ -536,6 +565,8 @@ int batch_advance(cfs_batch* b, int nsteps, double cfl, double dt, const double*
         p.dt_fixed = dt_case ? dt_case[ci] : dt;
     }
     CFSB_CUDA(b, cudaMemcpyAsync(b->P, hp.data(), sizeof(cfs::DevParams) * b->n, cudaMemcpyHostToDevice, b->stream));
+    // (the stages keep the counters at 0 among themselves; a call that failed half way may not have)
+    CFSB_CUDA(b, cudaMemsetAsync(b->counters, 0, sizeof(unsigned int) * cfs::kBatchCounters, b->stream));
     // first step's CFL maxima: the stage-0 arguments of parity 0 read S0 and
     // point at each case's parameters
     if (cfl > 0) CFSB_CUDA(b, cfs::launch_batch_wmax(b->elem, b->dargs, b->n, b->stream));

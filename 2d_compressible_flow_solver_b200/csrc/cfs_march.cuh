@@ -19,6 +19,7 @@
 // 172-178: both walkers stop, so interior slots repeat the first interior cell).
 #pragma once
 #include "cfs_kernels.cuh"
+#include "cfs_launch.h"
 
 namespace cfs {
 
@@ -1063,7 +1064,7 @@ template <class Pol, int kWarps, int kMinBlocks, int kLoad, int kFeat>
 __global__ void __launch_bounds__(32 * kWarps, kMinBlocks)
     batch_march_kernel(const StageArgs* __restrict__ args, const int* __restrict__ unit_case,
                        const int* __restrict__ unit_local, const int* __restrict__ case_rows,
-                       const int* __restrict__ case_nseg, int total, unsigned int* counter) {
+                       const int* __restrict__ case_nseg, int total, unsigned int* counters, int slot) {
     using C = typename Pol::C;
     __shared__ __align__(16) C rbuf[kWarps][36][kVars];
     constexpr bool kRing = kLoad == 3;
@@ -1072,6 +1073,9 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks)
     extern __shared__ __align__(128) unsigned char batch_dyn_smem[];
     typename Pol::T* const ring = kDynRing ? reinterpret_cast<typename Pol::T*>(batch_dyn_smem) : ring_static;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned int* const counter = counters + slot;
+    if (blockIdx.x == 0 && threadIdx.x < kBatchCounters && threadIdx.x / kBatchMaxGroups != slot / kBatchMaxGroups)
+        counters[threadIdx.x] = 0u;  // the other stages' (see kBatchCounters)
     C(&wbuf)[1][36][kVars] = *reinterpret_cast<C(*)[1][36][kVars]>(&rbuf[wid]);
     for (;;) {
         unsigned int w = 0u;

@@ -102,8 +102,8 @@ cudaError_t allow_dyn(Kernel k, size_t bytes) {
 
 template <class Pol, int kMinBlocks, int kLoad>
 cudaError_t launch_batch_march(const StageArgs* args, const int* item_case, const int* item_local,
-                               const int* case_rows, const int* case_nseg, int total, unsigned int* counter,
-                               int grid, int feat, cudaStream_t s) {
+                               const int* case_rows, const int* case_nseg, int total, unsigned int* counters,
+                               int slot, int grid, int feat, cudaStream_t s) {
     constexpr size_t dyn = batch_dyn_bytes<Pol, kLoad>();
     cudaError_t e = cudaSuccess;
     switch (feat) {
@@ -119,19 +119,19 @@ cudaError_t launch_batch_march(const StageArgs* args, const int* item_case, cons
     switch (feat) {
         case 0:
             batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, 0><<<grid, 32 * kBatchWarps, dyn, s>>>(
-                args, item_case, item_local, case_rows, case_nseg, total, counter);
+                args, item_case, item_local, case_rows, case_nseg, total, counters, slot);
             break;
         case kFeatPos:
             batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeatPos><<<grid, 32 * kBatchWarps, dyn, s>>>(
-                args, item_case, item_local, case_rows, case_nseg, total, counter);
+                args, item_case, item_local, case_rows, case_nseg, total, counters, slot);
             break;
         case kFeatEdge:
             batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeatEdge><<<grid, 32 * kBatchWarps, dyn, s>>>(
-                args, item_case, item_local, case_rows, case_nseg, total, counter);
+                args, item_case, item_local, case_rows, case_nseg, total, counters, slot);
             break;
         case kFeatEdge | kFeatPos:
             batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeatEdge | kFeatPos><<<grid, 32 * kBatchWarps, dyn, s>>>(
-                args, item_case, item_local, case_rows, case_nseg, total, counter);
+                args, item_case, item_local, case_rows, case_nseg, total, counters, slot);
             break;
         default:
             return cudaErrorInvalidValue;
@@ -140,14 +140,14 @@ cudaError_t launch_batch_march(const StageArgs* args, const int* item_case, cons
 }
 
 cudaError_t launch_batch_stage(Prec p, const StageArgs* args, const int* item_case, const int* item_local,
-                               const int* case_rows, const int* case_nseg, int total, unsigned int* counter,
-                               int grid, int feat, cudaStream_t s) {
+                               const int* case_rows, const int* case_nseg, int total, unsigned int* counters,
+                               int slot, int grid, int feat, cudaStream_t s) {
     if (total <= 0) return cudaSuccess;
     if (p == kF32Mixed)
         return launch_batch_march<PolF32, kBatchMinBlocksF32, kBatchLoadF32>(args, item_case, item_local, case_rows,
-                                                                             case_nseg, total, counter, grid, feat, s);
+                                                                             case_nseg, total, counters, slot, grid, feat, s);
     return launch_batch_march<PolF64, kBatchMinBlocksF64, kBatchLoadF64>(args, item_case, item_local, case_rows,
-                                                                         case_nseg, total, counter, grid, feat, s);
+                                                                         case_nseg, total, counters, slot, grid, feat, s);
 }
 
 // Boundary-face fluxes of every case of a batch (cases without Dirichlet sides
