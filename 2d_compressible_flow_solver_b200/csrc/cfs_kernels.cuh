@@ -423,20 +423,27 @@ __device__ __forceinline__ unsigned int cell_hash(int i, int j, unsigned int ste
                   step_seed * 0xc2b2ae3du);
 }
 
-// Dither of stochastic rounding for a result near f: uniform over one float
+// Dither of stochastic rounding for results near f: uniform over one float
 // spacing g of f's binade, (u + 1/2)/256 - 1/2 times g for the 8 random bits u
-// (the low byte of `bits`), built by placing u in the mantissa of a float in
-// [1, 2).  Added to a value x between neighbouring floats lo < x < lo + g
-// before one round-to-nearest, it picks lo + g with probability (x - lo)/g (to
-// 1/256).  Just below a power of two the spacing halves, so there the choice
-// is only approximately unbiased; for |f| below 2^-103 the dither is 0 (round
-// to nearest).
-__device__ __forceinline__ float sr_dither(float f, unsigned int bits) {
-    const int eb = static_cast<int>(__float_as_uint(f) & 0x7f800000u);
-    const float g = __int_as_float(max(eb - (23 << 23), 0));
-    const float m = __uint_as_float(0x3f800000u | ((bits & 255u) << 15) | (1u << 14));
-    return fmaf(m, g, -1.5f * g);
+// (a byte of `h`, one per variable).  Added to a value x between neighbouring
+// floats lo < x < lo + g before one round-to-nearest, it picks lo + g with
+// probability (x - lo)/g (to 1/256).  Just below a power of two the spacing
+// halves, so there the choice is only approximately unbiased; for |f| in the
+// subnormal range the dither is 0 (round to nearest).
+// Formed as the binade's power of two (f's exponent bits, 0 for f = 0) times
+// the byte's factor of 2^-23: one byte permutation puts u under the mantissa
+// of a float near 2^-16 (steps of 2^-31), and subtracting that float's centre
+// leaves (u + 1/2)/256 - 1/2 in units of 2^-23, exactly.  Two variables share
+// each packed subtraction and the multiply-add that adds the dither to the
+// increment: about 20 instructions per cell-stage fewer than shifting each byte
+// into a mantissa and scaling by an integer-built spacing, the 4096^2 step
+// 1,411 -> 1,384 us.
+__device__ __forceinline__ float binade(float f) { return __uint_as_float(__float_as_uint(f) & 0x7f800000u); }
+template <int kByte>
+__device__ __forceinline__ float dither_bits(unsigned int h) {
+    return __uint_as_float(__byte_perm(h, 0x37800080u, 0x7604u | (kByte << 4)));
 }
+constexpr float kDitherCentre = 257.0f / 16777216.0f;  // 2^-16 (1 + 2^-8), the middle of the 256 values
 
 // Positivity floors of CFS_POSITIVITY_FLOOR (no reference counterpart): a new
 // state with rho <= kRhoFloor (or a NaN) becomes the floor state at rest (the

@@ -822,14 +822,15 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
                         // spacing of the result's binade, and is added to x0 with
                         // one rounding; two variables per packed instruction.
                         const unsigned int h = cell_hash(i, j, step_seed);
+                        const float u[kVars] = {dither_bits<0>(h), dither_bits<1>(h), dither_bits<2>(h), dither_bits<3>(h)};
 #pragma unroll
                         for (int v = 0; v < kVars; v += 2) {
                             const float2 a0 = make_float2(x0[v], x0[v + 1]);
                             const float2 inc = fma2(p2(cB), sub2(make_float2(x1[v], x1[v + 1]), a0),
                                                     mul2(p2(cdt), make_float2(rvf[v], rvf[v + 1])));
                             const float2 f = add2(a0, inc);
-                            const float2 dz = make_float2(sr_dither(f.x, h >> (8 * v)), sr_dither(f.y, h >> (8 * v + 8)));
-                            const float2 r = add2(a0, add2(inc, dz));
+                            const float2 t = add2(make_float2(u[v], u[v + 1]), p2(-kDitherCentre));
+                            const float2 r = add2(a0, fma2(make_float2(binade(f.x), binade(f.y)), t, inc));
                             ndv[v] = r.x;
                             ndv[v + 1] = r.y;
                         }
