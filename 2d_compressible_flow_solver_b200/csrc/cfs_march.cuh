@@ -1015,13 +1015,17 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) march_kernel(const __
     const int nseg = (a.L.ny + kSeg - 1) / kSeg;
     const long long nitems =
         static_cast<long long>(nseg) * ((stage_row_hi(a) - stage_row_lo(a) + rows - 1) / rows);
-    const long long gw = static_cast<long long>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
+    // (the warp index taken from lane 0, so that the compiler knows the item's
+    // rows and columns to be the same in all lanes: the row tests' branches need
+    // no convergence code.  685 -> 670 instructions per cell-stage in FP32, the
+    // 4096^2 step 1,384 -> 1,356 us, 2048^2 FP64 689 -> 666)
+    const int wid = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+    const long long gw = static_cast<long long>(blockIdx.x) * kWarps + wid;
     const int seg = gw < nitems ? static_cast<int>(gw % nseg) : nseg;
     const int by = gw < nitems ? static_cast<int>(gw / nseg) : 0;
     // (the ring forms use no row buffer)
     __shared__ __align__(16) typename Pol::C rbuf[kLoad >= 3 ? 1 : kWarps][36][kVars];
     using RB = typename Pol::C(&)[kWarps][36][kVars];
-    const int wid = threadIdx.x >> 5;
     if constexpr (kLoad == 4) {
         __shared__ __align__(8) unsigned long long bars[kWarps][kRingRows];
         init_ring_bars<kWarps>(bars, wid);
@@ -1051,7 +1055,7 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) march_kernel(const __
         march_item<Pol, kWarps, kLoad, kFeat>(a, seg, by, rows, reinterpret_cast<RB>(rbuf),
                                               reinterpret_cast<typename Pol::T*>(march_dyn_smem), wid);
     } else {
-        march_item<Pol, kWarps, kLoad, kFeat>(a, seg, by, rows, rbuf, nullptr, threadIdx.x >> 5);
+        march_item<Pol, kWarps, kLoad, kFeat>(a, seg, by, rows, rbuf, nullptr, wid);
     }
 }
 
