@@ -230,27 +230,35 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // Ring of staged rows of the row march (load schedules 3 and 4), per warp:
 // kRingRows rows of its 36 columns (the segment and 2 halo columns each side,
-// whole cells), stored values, and (FP32 storage) the same 36 columns of the
-// rows of U^0 (lane l reads column l + 2).  The FP64 ring leaves U^0 out (each
-// lane loads it early in the row's iteration): its rows of doubles would
-// otherwise cost a fourth block per SM.
-// A ring row holds 36 cells and starts 128-byte aligned, as a TMA copy's
-// shared-memory destination must: its stride is rounded up to 128 bytes
-// (FP32: 576 bytes of cells in a 640-byte row; FP64: 1,152 bytes, already a
-// multiple).
+// whole cells), stored values, and (FP32 storage) the rows of U^0.  The FP64
+// ring leaves U^0 out (each lane loads it early in the row's iteration): its
+// rows of doubles would otherwise cost a fourth block per SM.
+//
+// cp.async (schedule 3): rows packed (576 / 1,152 bytes), U^0 rows of the 32
+// lanes' own columns.  (Keeping the first four slots once more behind the
+// last, so that an x-stencil's five rows are immediate offsets from one
+// address, takes 27 instructions per cell-stage less but lost: 1,329 against
+// 1,317 us for the 4096^2 step, FP64 677 against 647 at 2048^2; the ring then
+// takes all of the SM's shared memory.)
+//
+// TMA (schedule 4): one box per row; a row starts 128-byte
+// aligned, as a TMA copy's shared-memory destination must (its stride rounded
+// up to 128 bytes: FP32 640, FP64 1,152), U^0 rows alike.
 constexpr int kRingRows = 8, kRingDist = 2;
 constexpr int kRingCols = 36;
 template <class T>
 __host__ __device__ constexpr int ring_row_words() {
     return ((kRingCols * kVars * static_cast<int>(sizeof(T)) + 127) / 128) * 128 / static_cast<int>(sizeof(T));
 }
-template <class T>
+template <class T, int kLoad>
 __host__ __device__ constexpr int ring_words() {
-    return sizeof(T) == 4 ? kRingRows * 2 * ring_row_words<T>() : kRingRows * ring_row_words<T>();
+    if (kLoad == 3) return kRingRows * (kRingCols + (sizeof(T) == 4 ? 32 : 0)) * kVars;
+    return (sizeof(T) == 4 ? 2 : 1) * kRingRows * ring_row_words<T>();
 }
 static_assert(ring_row_words<float>() * 4 % 128 == 0 && ring_row_words<double>() * 8 % 128 == 0,
-              "ring rows start 128-byte aligned");
-static_assert(ring_words<float>() * 4 % 128 == 0 && ring_words<double>() * 8 % 128 == 0,
+              "TMA ring rows start 128-byte aligned");
+static_assert(ring_words<float, 4>() * 4 % 128 == 0 && ring_words<double, 4>() * 8 % 128 == 0 &&
+                  ring_words<float, 3>() * 4 % 128 == 0 && ring_words<double, 3>() * 8 % 128 == 0,
               "each warp's ring starts 128-byte aligned");
 
 // ---- TMA staging (load schedule 4).  One elected lane of a warp copies a
@@ -609,16 +617,35 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
         if (a.stage >= 1) ld_cell<T>(static_cast<const T*>(a.u0), off, pf_u0);
     };
 
-    // Load schedule 3: this warp's ring (rows, and U^0 rows in FP32; ring_words).
+    // Load schedules 3, 4: this warp's ring (rows, and U^0 rows in FP32; ring_words).
     constexpr bool kU0Ring = kRing && sizeof(T) == 4;
-    constexpr int kRowWords = ring_row_words<T>();
-    T* const rw = kRing ? ring + wid * ring_words<T>() : nullptr;
-    T* const ru0 = kU0Ring ? rw + kRingRows * kRowWords : nullptr;
+    constexpr int kRowWords = kTma ? ring_row_words<T>() : kRingCols * kVars;
+    constexpr int kU0Words = kTma ? ring_row_words<T>() : 32 * kVars;
+    T* const rw = kRing ? ring + wid * ring_words<T, kLoad>() : nullptr;
+    T* const ru0 = kU0Ring ? rw + kRingRows * kRowWords + (kTma ? 2 * kVars : 0) : nullptr;
     auto ring_row = [&](int q) -> T* { return rw + (q & (kRingRows - 1)) * kRowWords; };
-    auto ring_u0 = [&](int q) -> T* { return ru0 + (q & (kRingRows - 1)) * kRowWords; };
-    // Issue the copies of row q (the lane's column; halo lanes also their
-    // halo column) and, for an updated row, of its U^0; one commit group per
-    // row (empty past the last row needed, so group counts stay uniform).
+    auto ring_u0 = [&](int q) -> T* { return ru0 + (q & (kRingRows - 1)) * kU0Words; };
+    // cp.async: ring column c is cell j0 - 3 + c; a lane copies columns lane
+    // and (lanes 0..3) 32 + lane, and its own column of U^0, from pointers that
+    // step one row per issued row; a column past the padded row is zero filled
+    // from column 0's address.  (Addresses formed from row and column for each
+    // copy, with the halo columns on lanes 0, 1, 30 and 31, took 30 more
+    // instructions per cell-stage: SSP3 step of 4096^2 FP32-mixed 1,356 ->
+    // 1,308 us, 2048^2 FP64 666 -> 647.)
+    const bool src_ok = j0 - 3 + lane <= L.ny + kGhost - 1, src2_ok = j0 + 29 + lane <= L.ny + kGhost - 1;
+    const T* src = nullptr;
+    const T* src2 = nullptr;
+    const T* src_u0 = nullptr;
+    const long long row_step = static_cast<long long>(L.pitch) * kVars;
+    const int u0_rows = a.stage >= 1 ? i1 - i0 : 0;  // rows whose U^0 is staged, from i0
+    if constexpr (kLoad == 3) {
+        src = in + Layout::at(L.offset(i0 - 3, src_ok ? j0 - 3 + lane : 0), 0);
+        src2 = in + Layout::at(L.offset(i0 - 3, src2_ok ? j0 + 29 + lane : 0), 0);
+        if (kU0Ring) src_u0 = static_cast<const T*>(a.u0) + Layout::at(L.offset(i0 - 3, col_ok ? j : 0), 0);
+    }
+    // Issue the copies of row q and, for an updated row, of its U^0; one commit
+    // group per row (empty past the last row needed, so group counts stay
+    // uniform).
     // TMA: lane 0 copies the row's 36 cells (and U^0's) as one box each,
     // completing on the slot's mbarrier.
     constexpr unsigned kRowBytes = kRingCols * kVars * sizeof(T);
@@ -631,7 +658,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
             if (lane == 0) {
                 const bool u0row = kU0Ring && a.stage >= 1 && q >= i0 && q < i1;
                 const unsigned bar = smem_addr(bars + (q & (kRingRows - 1)));
-                const unsigned dst = smem_addr(ring_row(q)), dst0 = u0row ? smem_addr(ring_u0(q)) : 0u;
+                const unsigned dst = smem_addr(ring_row(q)), dst0 = u0row ? smem_addr(ring_u0(q) - 2 * kVars) : 0u;
                 if (((dst | dst0) & 127u) != 0u) {
                     // self-check: never issue a copy to a misaligned row;
                     // complete the slot's phase without data and flag it
@@ -646,20 +673,15 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
             }
         } else if constexpr (kRing) {
             if (q <= i1 + 2) {
-                T* dst = ring_row(q);
-                const long long off = L.offset(q, col_ok ? j : 0);
-                cp_async_cell<T>(dst + (lane + 2) * kVars, in + Layout::at(off, 0), col_ok);
-                if (lane < 2 || lane >= 30) {
-                    const int hc = lane < 2 ? j0 - 3 + lane : j0 + 1 + lane;
-                    const bool ok = hc <= L.ny + kGhost - 1;
-                    const long long hoff = L.offset(q, ok ? hc : 0);
-                    const int slot = lane < 2 ? lane : lane + 4;
-                    cp_async_cell<T>(dst + slot * kVars, in + Layout::at(hoff, 0), ok);
-                }
-                if (kU0Ring && a.stage >= 1 && q >= i0 && q < i1)  // uniform: every lane fills its slot
-                    cp_async_cell<T>(ring_u0(q) + (lane + 2) * kVars, static_cast<const T*>(a.u0) + Layout::at(off, 0),
-                                     col_ok);
+                T* const dst = ring_row(q) + lane * kVars;
+                cp_async_cell<T>(dst, src, src_ok);
+                if (lane < 4) cp_async_cell<T>(dst + 32 * kVars, src2, src2_ok);
+                if (kU0Ring && static_cast<unsigned>(q - i0) < static_cast<unsigned>(u0_rows))
+                    cp_async_cell<T>(ring_u0(q) + lane * kVars, src_u0, col_ok);
             }
+            src += row_step;
+            src2 += row_step;
+            if (kU0Ring) src_u0 += row_step;
             cp_async_commit();
         }
     };
@@ -739,9 +761,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
             }
 #pragma unroll
             for (int k = 0; k < 5; ++k) {  // stored deviations; offsets added after the reconstruction
-                const T* src = ring_row(r - 2 + k) + (lane + 2) * kVars;
-#pragma unroll
-                for (int v = 0; v < kVars; ++v) win[k][v] = C(src[v]);
+                ld_cell<T>(ring_row(r - 2 + k), lane + 2, win[k]);
             }
         }
         if constexpr (kL == 2) {
@@ -783,13 +803,11 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
             if (i >= i0 && owner) {
                 if constexpr (kRing) {
                     const T* cs = ring_row(i) + (lane + 2) * kVars;
-#pragma unroll
-                    for (int v = 0; v < kVars; ++v) pf_cur[v] = cs[v];
+                    ld_cell<T>(cs, 0, pf_cur);
                     if constexpr (kU0Ring) {
                         // U^0 (stage 0: the current state, the update's x0 then)
-                        const T* us = (a.stage >= 1 ? ring_u0(i) : ring_row(i)) + (lane + 2) * kVars;
-#pragma unroll
-                        for (int v = 0; v < kVars; ++v) pf_u0[v] = us[v];
+                        const T* us = a.stage >= 1 ? ring_u0(i) + lane * kVars : cs;
+                        ld_cell<T>(us, 0, pf_u0);
                     }
                 } else if constexpr (kL == 0) {
                     load_update(i);
@@ -893,9 +911,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
             if constexpr (kRing) {
                 const T* row = ring_row(r);
 #pragma unroll
-                for (int k = 0; k < 5; ++k)
-#pragma unroll
-                    for (int v = 0; v < kVars; ++v) st[k][v] = C(row[(lane + k) * kVars + v]);  // deviations
+                for (int k = 0; k < 5; ++k) ld_cell<T>(row, lane + k, st[k]);  // deviations
             } else {
                 C(*rb)[kVars] = rbuf[wid];
                 put_slot<C>(rb[lane + 2], win[2]);
@@ -1035,7 +1051,7 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) march_kernel(const __
         }
         unsigned phase = 0u;
         if constexpr (sizeof(typename Pol::T) == 4) {
-            __shared__ __align__(128) typename Pol::T ring[kWarps * ring_words<typename Pol::T>()];
+            __shared__ __align__(128) typename Pol::T ring[kWarps * ring_words<typename Pol::T, kLoad>()];
             march_item<Pol, kWarps, kLoad, kFeat>(a, seg, by, rows, reinterpret_cast<RB>(rbuf), ring, wid,
                                                   bars[wid], &phase);
         } else {
@@ -1046,10 +1062,10 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) march_kernel(const __
                                                   &phase);
         }
     } else if constexpr (kLoad == 3 && sizeof(typename Pol::T) == 4) {
-        __shared__ __align__(128) typename Pol::T ring[kWarps * ring_words<typename Pol::T>()];
+        __shared__ __align__(128) typename Pol::T ring[kWarps * ring_words<typename Pol::T, kLoad>()];
         march_item<Pol, kWarps, kLoad, kFeat>(a, seg, by, rows, reinterpret_cast<RB>(rbuf), ring, wid);
     } else if constexpr (kLoad == 3) {
-        // FP64 ring: kWarps * ring_words<double>() doubles (36.9 KB for 4
+        // FP64 ring: kWarps * ring_words<double, 3>() doubles (36.9 KB for 4
         // warps); dynamic shared memory, sized at launch
         extern __shared__ __align__(128) unsigned char march_dyn_smem[];
         march_item<Pol, kWarps, kLoad, kFeat>(a, seg, by, rows, reinterpret_cast<RB>(rbuf),
@@ -1071,17 +1087,17 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks)
                        const int* __restrict__ unit_local, const int* __restrict__ case_rows,
                        const int* __restrict__ case_nseg, int total, unsigned int* counters, int slot) {
     using C = typename Pol::C;
-    __shared__ __align__(16) C rbuf[kWarps][36][kVars];
     constexpr bool kRing = kLoad == 3;
+    __shared__ __align__(16) C rbuf[kRing ? 1 : kWarps][36][kVars];  // (the ring forms use no row buffer)
     constexpr bool kDynRing = kRing && sizeof(typename Pol::T) == 8;  // FP64: ring in dynamic shared memory
-    __shared__ __align__(128) typename Pol::T ring_static[kRing && !kDynRing ? kWarps * ring_words<typename Pol::T>() : 1];
+    __shared__ __align__(128) typename Pol::T ring_static[kRing && !kDynRing ? kWarps * ring_words<typename Pol::T, kLoad>() : 1];
     extern __shared__ __align__(128) unsigned char batch_dyn_smem[];
     typename Pol::T* const ring = kDynRing ? reinterpret_cast<typename Pol::T*>(batch_dyn_smem) : ring_static;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     unsigned int* const counter = counters + slot;
     if (blockIdx.x == 0 && threadIdx.x < kBatchCounters && threadIdx.x / kBatchMaxGroups != slot / kBatchMaxGroups)
         counters[threadIdx.x] = 0u;  // the other stages' (see kBatchCounters)
-    C(&wbuf)[1][36][kVars] = *reinterpret_cast<C(*)[1][36][kVars]>(&rbuf[wid]);
+    C(&wbuf)[1][36][kVars] = *reinterpret_cast<C(*)[1][36][kVars]>(&rbuf[kRing ? 0 : wid]);
     for (;;) {
         unsigned int w = 0u;
         if (lane == 0) w = atomicAdd(counter, 1u);
@@ -1090,7 +1106,7 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks)
         const int c = unit_case[w], lu = unit_local[w];
         const int ns = case_nseg[c];
         const StageArgs a = args[c];
-        march_item<Pol, 1, kLoad, kFeat>(a, lu % ns, lu / ns, case_rows[c], wbuf, kRing ? ring + wid * ring_words<typename Pol::T>() : nullptr, 0);
+        march_item<Pol, 1, kLoad, kFeat>(a, lu % ns, lu / ns, case_rows[c], wbuf, kRing ? ring + wid * ring_words<typename Pol::T, kLoad>() : nullptr, 0);
     }
 }
 

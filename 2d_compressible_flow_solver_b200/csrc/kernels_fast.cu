@@ -91,7 +91,7 @@ cudaError_t launch_stage_f32(const StageArgs& a, cudaStream_t s) {
 // Dynamic shared memory of a batched march (the FP64 ring), 0 for the others.
 template <class Pol, int kLoad>
 constexpr size_t batch_dyn_bytes() {
-    return (kLoad == 3 && sizeof(typename Pol::T) == 8) ? static_cast<size_t>(kBatchWarps) * ring_words<double>() * 8 : 0;
+    return (kLoad == 3 && sizeof(typename Pol::T) == 8) ? static_cast<size_t>(kBatchWarps) * ring_words<double, kLoad>() * 8 : 0;
 }
 
 template <class Kernel>

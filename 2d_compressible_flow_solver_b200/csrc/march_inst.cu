@@ -33,7 +33,7 @@ cudaError_t launch_march(const StageArgs& a_in, cudaStream_t s) {
         // on one device at the same time)
         static std::once_flag once[kMaxDev];
         static cudaError_t allow_err[kMaxDev];
-        dyn = static_cast<size_t>(W) * ring_words<double>() * sizeof(double);
+        dyn = static_cast<size_t>(W) * ring_words<double, Ld>() * sizeof(double);
         auto allow = [dyn] {
             return cudaFuncSetAttribute(march_kernel<Pol, R, W, B, Ld, F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(dyn));
