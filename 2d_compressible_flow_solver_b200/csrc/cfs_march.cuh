@@ -116,29 +116,31 @@ __device__ __forceinline__ void weno5_pair_x2(float2 v0, float2 v1, float2 v2, f
     right = fma2(fma2(Z5, B0, fma2(Y, B1, mul2(X, B2))), iR, v2);
 }
 
-// finish_state of a cell's two states at once (FP32-mixed: packed
-// instructions; a state whose kinetic energy exceeds 90 % of E takes the scalar
-// path with its FP64 pressure).
+// finish_state of a cell's two states at once (FP32-mixed: a state whose
+// kinetic energy exceeds 90 % of E takes the FP64 path of finish_state).
+// Scalar: the packed form did the same operations in half the instructions
+// but moved eight values into register pairs first, and a packed operation
+// keeps the FMA pipe busy as long as two scalar ones.  With ke = m^2 / rho / 2
+// and t = E - ke: p = (g - 1) t, a = sqrt(g (g - 1) t / rho).
 template <class Pol>
 __device__ __forceinline__ void finish_pair(Face5<typename Pol::C>& L, Face5<typename Pol::C>& R, double g) {
     if constexpr (Pol::kMixed) {
-        const float2 mx = make_float2(L.mx, R.mx), my = make_float2(L.my, R.my), E = make_float2(L.E, R.E);
-        const float2 ri = make_float2(rcp_fast(L.r), rcp_fast(R.r));
-        const float2 ke = mul2(mul2(p2(0.5f), fma2(mx, mx, mul2(my, my))), ri);
-        if (ke.x > 0.9f * L.E || ke.y > 0.9f * R.E) {
+        const float gm1 = float(g - 1), gg = float(g) * float(g - 1);
+        const float riL = rcp_fast(L.r), riR = rcp_fast(R.r);
+        const float tL = fmaf(-0.5f, fmaf(L.mx, L.mx, L.my * L.my) * riL, L.E);
+        const float tR = fmaf(-0.5f, fmaf(R.mx, R.mx, R.my * R.my) * riR, R.E);
+        if (tL < 0.1f * L.E || tR < 0.1f * R.E) {
             finish_state<Pol>(L, g);
             finish_state<Pol>(R, g);
             return;
         }
-        const float2 p = mul2(p2(float(g - 1)), sub2(E, ke));
-        const float2 a2 = mul2(mul2(p2(float(g)), p), ri);
-        const float2 a = mul2(a2, make_float2(rsqrt_fast(a2.x), rsqrt_fast(a2.y)));
-        L.ri = ri.x;
-        R.ri = ri.y;
-        L.p = p.x;
-        R.p = p.y;
-        L.a = a.x;
-        R.a = a.y;
+        const float a2L = gg * tL * riL, a2R = gg * tR * riR;
+        L.ri = riL;
+        R.ri = riR;
+        L.p = gm1 * tL;
+        R.p = gm1 * tR;
+        L.a = a2L * rsqrt_fast(a2L);
+        R.a = a2R * rsqrt_fast(a2R);
     } else {
         finish_state<Pol>(L, g);
         finish_state<Pol>(R, g);
