@@ -120,7 +120,8 @@ __device__ __forceinline__ void weno5_pair_x2(float2 v0, float2 v1, float2 v2, f
 // kinetic energy exceeds 90 % of E takes the FP64 path of finish_state).
 // Scalar: the packed form did the same operations in half the instructions
 // but moved eight values into register pairs first, and a packed operation
-// keeps the FMA pipe busy as long as two scalar ones.  With ke = m^2 / rho / 2
+// keeps the FMA pipe busy as long as two scalar ones (4096^2 step 1,308 ->
+// 1,278 us).  With ke = m^2 / rho / 2
 // and t = E - ke: p = (g - 1) t, a = sqrt(g (g - 1) t / rho).
 template <class Pol>
 __device__ __forceinline__ void finish_pair(Face5<typename Pol::C>& L, Face5<typename Pol::C>& R, double g) {
