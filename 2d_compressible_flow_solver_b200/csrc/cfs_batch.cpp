@@ -222,6 +222,9 @@ int enqueue_batch_step(cfs_batch* b, int parity) {
     for (int s = 0; s < S; ++s) {
         const int slot = parity * 3 + s;
         const int in = s;  // stage s reads S_s (S0, S1, S2)
+        const int scheme = cfs::known_scheme(
+            b->common.hll == CFS_HLL_DAVIS, b->common.rk == CFS_RK_TVD3_REFERENCE, s,
+            b->prec != cfs::kF32Mixed || cfs::stage_rounds_stochastically(b->common.rounding, s == S - 1));
         if (b->total_ig > 0)
             CFSB_CUDA(b, cfs::launch_batch_ib_fill(b->elem, b->dib + static_cast<size_t>(in) * b->n, b->ig_case,
                                                    b->ig_local, b->total_ig, b->stream));
@@ -233,7 +236,7 @@ int enqueue_batch_step(cfs_batch* b, int parity) {
             CFSB_CUDA(b, cfs::launch_batch_stage(b->prec, b->dargs + static_cast<size_t>(slot) * b->n,
                                                  b->item_case + fg.first, b->item_local + fg.first, b->case_rows,
                                                  b->case_nseg, fg.count, b->counters, slot * cfs::kBatchMaxGroups + static_cast<int>(g),
-                                                 b->grid, fg.feat, b->stream));
+                                                 b->grid, fg.feat, scheme, b->stream));
         }
     }
     return CFS_OK;

@@ -69,11 +69,6 @@ constexpr MarchVariant kVariants[kNumVariants] = {
 // 4,448).
 constexpr int kDefaultVariantF32 = 7;
 constexpr int kDefaultVariantF64 = 8;
-// FP32 grids with edge code (physical sides, cell types) run the same ring
-// march with 128 registers and 4 blocks per SM: 2048^2 transmissive with floors
-// and a cylinder 5,672 against 5,476 Mcell-steps/s, the 2048 x 1024 Mach-3
-// cylinder 5,237 against 5,039.
-constexpr int kEdgeVariantF32 = 8;
 // FP64 ring blocks per SM (4 warps at 128 registers; 37 KB dynamic + 4.6 KB
 // static shared memory), and the register-window variant the FP64 default
 // falls back to when the ring's last wave would run nearly empty
@@ -137,7 +132,8 @@ constexpr int kBatchMaxGroups = 4;  // the feature sets a batch launches: 0, Pos
 constexpr int kBatchCounters = 2 * 3 * kBatchMaxGroups;
 cudaError_t launch_batch_stage(Prec p, const StageArgs* args, const int* item_case, const int* item_local,
                                const int* case_rows, const int* case_nseg, int total, unsigned int* counters,
-                               int slot, int grid, int feat, cudaStream_t s);  // feat: kFeatPos | kFeatEdge bits
+                               int slot, int grid, int feat, int scheme,
+                               cudaStream_t s);  // feat: kFeatPos | kFeatEdge bits; scheme: known_scheme
 // Boundary-face fluxes of every case (grid: max_edge = the largest nx or ny).
 cudaError_t launch_batch_boundary_flux(Prec p, const StageArgs* args, int ncases, int max_edge, cudaStream_t s);
 cudaError_t launch_batch_ib_fill(int elem_bytes, const IbArgs* args, const int* cases, const int* local, int total,

@@ -157,6 +157,27 @@ CFS_HD bool dirichlet_side(const int bc[4]) {
 constexpr int kFeatPos = 1;    // positivity fallbacks and floors (StageArgs::positivity != 0)
 constexpr int kFeatExtra = 2;  // RHS copy (StageArgs::rhs) and viscous RHS (StageArgs::rv)
 constexpr int kFeatEdge = 4;   // physical sides or cell flags (StageArgs::cflags)
+// A launch's scheme, fixed at compile time for the variants that run by default
+// (kScheme* bits beside the features): the HLL bounds, whether the stage reads
+// U^1 (TVD3 as written, its last stage), and that it rounds stochastically
+// (FP32 storage).  Tested at run time these cost uniform branches that split
+// the row body into pieces the compiler does not schedule across: SSP3 + Davis
+// 4096^2 FP32-mixed 1,278 -> 1,242 us a step, the 2048 x 1024 cylinder 281 -> 259, the
+// uneven batch 950 -> 901, 2048^2 FP64 647 -> 630.
+// Launches outside the three combinations (0) test them at run time.
+constexpr int kSchemeDavis = 8, kSchemeHllRef = 16, kSchemeU1 = 32, kSchemeNoU1 = 64, kSchemeSr = 128;
+constexpr int kScheme0 = kSchemeDavis | kSchemeNoU1 | kSchemeSr, kScheme1 = kSchemeHllRef | kSchemeNoU1 | kSchemeSr,
+              kScheme2 = kSchemeHllRef | kSchemeU1 | kSchemeSr;
+CFS_HD int known_scheme(int hll_davis, int rk_tvd3_ref, int stage, bool rounds_stochastically) {
+    const bool u1 = rk_tvd3_ref && stage == 2;
+    if (!rounds_stochastically || (hll_davis && u1)) return 0;
+    return hll_davis ? kScheme0 : u1 ? kScheme2 : kScheme1;
+}
+// FP32 storage: whether a stage rounds its new state stochastically.
+CFS_HD bool stage_rounds_stochastically(int rounding, bool last_of_step) {
+    return rounding == 2 || (rounding == 0 && last_of_step);
+}
+
 CFS_HD int march_features(const StageArgs& a) {
     bool edge = a.cflags != nullptr;
     for (int s = 0; s < 4; ++s) edge = edge || physical_side(a, s);

@@ -514,6 +514,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
     constexpr bool kPos = (kFeat & kFeatPos) != 0;
     constexpr bool kExtra = (kFeat & kFeatExtra) != 0;
     constexpr bool kEdge = (kFeat & kFeatEdge) != 0;
+    const int hll = (kFeat & kSchemeDavis) ? kHllDavis : (kFeat & kSchemeHllRef) ? kHllReference : a.hll;
     const Layout& L = a.L;
     const int lane = threadIdx.x & 31;
     const int j0 = seg * kSeg;
@@ -546,6 +547,8 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
         cdtd = (2.0 / 3.0) * dt;
         x1_u1 = a.rk == kRkTvd3Ref;
     }
+    if (kFeat & kSchemeU1) x1_u1 = true;
+    if (kFeat & kSchemeNoU1) x1_u1 = false;
     const float cdt = float(cdtd);
     // Stochastic rounding of the state that ends each step (the last stage), or
     // of every stage (CFS_ROUND_STOCHASTIC_ALL); otherwise round to nearest.
@@ -553,7 +556,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
     // increments are dt times differences of FP32 fluxes, a coarse lattice on
     // the stored grid, so the rounding errors do not average out.
     const bool last_of_step = a.rk == kRkTvd2 ? a.stage == 1 : a.stage == 2;
-    const bool sr = Pol::kMixed && ((a.rounding == 0 && last_of_step) || a.rounding == 2);
+    const bool sr = Pol::kMixed && ((kFeat & kSchemeSr) || stage_rounds_stochastically(a.rounding, last_of_step));
     const unsigned int step_seed = (a.P ? a.P->seed[a.parity] : a.seed) * 4u + static_cast<unsigned int>(a.stage);
     // physical boundary faces: the cell's own flux (transmissive) or a precomputed one (Dirichlet)
     const bool lo_x = kEdge && physical_side(a, 0), hi_x = kEdge && physical_side(a, 1);
@@ -787,7 +790,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
         if (r >= i0) {
             // (computed on a boundary row too and replaced there: a flux in a
             // branch of its own would not overlap the surrounding work)
-            hll_flux<Pol>(Lx, Rr, 0, a.hll, g, FX);
+            hll_flux<Pol>(Lx, Rr, 0, hll, g, FX);
             if ((r == 0 && lo_x) || (r == L.nx && hi_x)) {  // uniform per warp
                 // (no side index computed at run time: it would put the batch's argument block into local memory)
                 if (r == 0 ? a.bc[0] == kNeumann : a.bc[1] == kNeumann) {
@@ -818,7 +821,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
                 const bool fluid = !kEdge || !(f_prev & kCellSolid);
                 T* out = static_cast<T*>(a.out);
                 T u1c[kVars] = {T(0), T(0), T(0), T(0)};  // U^1 (TVD3 as written, stage 2 only)
-                if (a.stage == 2 && a.rk == kRkTvd3Ref) ld_cell<T>(static_cast<const T*>(a.u1), L.offset(i, j), u1c);
+                if (x1_u1) ld_cell<T>(static_cast<const T*>(a.u1), L.offset(i, j), u1c);
                 C nv[kVars];  // new state in the form's arithmetic type, for the CFL maximum
                 T sv[kVars];
                 if constexpr (Pol::kMixed) {
@@ -875,7 +878,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
                         if (kExtra && rv_in && v >= 1) rv += double(rv_cur[v - 1]);
                         const double cur = double(win[1][v]);
                         const double u0v = a.stage >= 1 ? dec<T>(pf_u0[v], L, v) : 0.0;
-                        const double u1v = (a.stage == 2 && a.rk == kRkTvd3Ref) ? dec<T>(u1c[v], L, v) : 0.0;
+                        const double u1v = x1_u1 ? dec<T>(u1c[v], L, v) : 0.0;
                         const double val = fluid ? rk_update(a.rk, a.stage, dt, cur, u0v, u1v, rv) : cur;
                         sv[v] = enc<T>(val, L, v);
                         nv[v] = C(dec<T>(sv[v], L, v));
@@ -942,7 +945,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
             Rn.ri = __shfl_down_sync(0xffffffffu, Ry.ri, 1);
             // face between column j and j+1 (face index j+1)
             C FY[kVars];
-            hll_flux<Pol>(Ly, Rn, 1, a.hll, g, FY);
+            hll_flux<Pol>(Ly, Rn, 1, hll, g, FY);
             if (warp_ybnd && ybnd) {
                 if (bfy) {
 #pragma unroll

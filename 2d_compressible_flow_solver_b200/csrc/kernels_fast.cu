@@ -72,7 +72,7 @@ cudaError_t launch_stage_f64(const StageArgs& a, cudaStream_t s) {
 cudaError_t launch_stage_f32(const StageArgs& a, cudaStream_t s) {
     const cudaError_t e = launch_boundary_flux<PolF32>(a, s);
     if (e != cudaSuccess) return e;
-    const int v = a.variant > 0 ? a.variant : (march_features(a) & kFeatEdge) ? kEdgeVariantF32 : kDefaultVariantF32;
+    const int v = a.variant > 0 ? a.variant : kDefaultVariantF32;
     switch (march_features(a)) {
         case 0: return launch_march_f32_0(a, v, s);
         case 1: return launch_march_f32_1(a, v, s);
@@ -100,54 +100,49 @@ cudaError_t allow_dyn(Kernel k, size_t bytes) {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
 }
 
-template <class Pol, int kMinBlocks, int kLoad>
-cudaError_t launch_batch_march(const StageArgs* args, const int* item_case, const int* item_local,
-                               const int* case_rows, const int* case_nseg, int total, unsigned int* counters,
-                               int slot, int grid, int feat, cudaStream_t s) {
+template <class Pol, int kMinBlocks, int kLoad, int kFeat>
+cudaError_t launch_batch_kernel(const StageArgs* args, const int* item_case, const int* item_local, const int* case_rows,
+                                const int* case_nseg, int total, unsigned int* counters, int slot, int grid,
+                                cudaStream_t s) {
     constexpr size_t dyn = batch_dyn_bytes<Pol, kLoad>();
-    cudaError_t e = cudaSuccess;
+    const cudaError_t e = allow_dyn(batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeat>, dyn);
+    if (e != cudaSuccess) return e;
+    batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeat><<<grid, 32 * kBatchWarps, dyn, s>>>(
+        args, item_case, item_local, case_rows, case_nseg, total, counters, slot);
+    return cudaGetLastError();
+}
+
+template <class Pol, int kMinBlocks, int kLoad, int kScheme, class... Args>
+cudaError_t launch_batch_feat(int feat, Args... args) {
     switch (feat) {
-        case 0: e = allow_dyn(batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, 0>, dyn); break;
-        case kFeatPos: e = allow_dyn(batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeatPos>, dyn); break;
-        case kFeatEdge: e = allow_dyn(batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeatEdge>, dyn); break;
+        case 0: return launch_batch_kernel<Pol, kMinBlocks, kLoad, kScheme>(args...);
+        case kFeatPos: return launch_batch_kernel<Pol, kMinBlocks, kLoad, kFeatPos | kScheme>(args...);
+        case kFeatEdge: return launch_batch_kernel<Pol, kMinBlocks, kLoad, kFeatEdge | kScheme>(args...);
         case kFeatEdge | kFeatPos:
-            e = allow_dyn(batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeatEdge | kFeatPos>, dyn);
-            break;
+            return launch_batch_kernel<Pol, kMinBlocks, kLoad, kFeatEdge | kFeatPos | kScheme>(args...);
         default: return cudaErrorInvalidValue;
     }
-    if (e != cudaSuccess) return e;
-    switch (feat) {
-        case 0:
-            batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, 0><<<grid, 32 * kBatchWarps, dyn, s>>>(
-                args, item_case, item_local, case_rows, case_nseg, total, counters, slot);
-            break;
-        case kFeatPos:
-            batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeatPos><<<grid, 32 * kBatchWarps, dyn, s>>>(
-                args, item_case, item_local, case_rows, case_nseg, total, counters, slot);
-            break;
-        case kFeatEdge:
-            batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeatEdge><<<grid, 32 * kBatchWarps, dyn, s>>>(
-                args, item_case, item_local, case_rows, case_nseg, total, counters, slot);
-            break;
-        case kFeatEdge | kFeatPos:
-            batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeatEdge | kFeatPos><<<grid, 32 * kBatchWarps, dyn, s>>>(
-                args, item_case, item_local, case_rows, case_nseg, total, counters, slot);
-            break;
-        default:
-            return cudaErrorInvalidValue;
+}
+
+template <class Pol, int kMinBlocks, int kLoad, class... Args>
+cudaError_t launch_batch_scheme(int scheme, int feat, Args... args) {
+    switch (scheme) {
+        case kScheme0: return launch_batch_feat<Pol, kMinBlocks, kLoad, kScheme0>(feat, args...);
+        case kScheme1: return launch_batch_feat<Pol, kMinBlocks, kLoad, kScheme1>(feat, args...);
+        case kScheme2: return launch_batch_feat<Pol, kMinBlocks, kLoad, kScheme2>(feat, args...);
+        default: return launch_batch_feat<Pol, kMinBlocks, kLoad, 0>(feat, args...);
     }
-    return cudaGetLastError();
 }
 
 cudaError_t launch_batch_stage(Prec p, const StageArgs* args, const int* item_case, const int* item_local,
                                const int* case_rows, const int* case_nseg, int total, unsigned int* counters,
-                               int slot, int grid, int feat, cudaStream_t s) {
+                               int slot, int grid, int feat, int scheme, cudaStream_t s) {
     if (total <= 0) return cudaSuccess;
     if (p == kF32Mixed)
-        return launch_batch_march<PolF32, kBatchMinBlocksF32, kBatchLoadF32>(args, item_case, item_local, case_rows,
-                                                                             case_nseg, total, counters, slot, grid, feat, s);
-    return launch_batch_march<PolF64, kBatchMinBlocksF64, kBatchLoadF64>(args, item_case, item_local, case_rows,
-                                                                         case_nseg, total, counters, slot, grid, feat, s);
+        return launch_batch_scheme<PolF32, kBatchMinBlocksF32, kBatchLoadF32>(
+            scheme, feat, args, item_case, item_local, case_rows, case_nseg, total, counters, slot, grid, s);
+    return launch_batch_scheme<PolF64, kBatchMinBlocksF64, kBatchLoadF64>(
+        scheme, feat, args, item_case, item_local, case_rows, case_nseg, total, counters, slot, grid, s);
 }
 
 // Boundary-face fluxes of every case of a batch (cases without Dirichlet sides

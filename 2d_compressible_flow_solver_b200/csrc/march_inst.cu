@@ -95,12 +95,27 @@ cudaError_t launch_march_k(const StageArgs& a, cudaStream_t s) {
     return launch_march<Pol, v.rows, v.warps, v.min_blocks, v.load, F>(a, s);
 }
 
+// The variant that runs by default, with the launch's scheme compiled in.
+template <class Pol, int K, int F>
+cudaError_t launch_march_default(const StageArgs& a, cudaStream_t s) {
+    const bool last_of_step = a.stage == (a.rk == kRkTvd2 ? 1 : 2);
+    const bool sr = !Pol::kMixed || stage_rounds_stochastically(a.rounding, last_of_step);
+    switch (known_scheme(a.hll == kHllDavis, a.rk == kRkTvd3Ref, a.stage, sr)) {
+        case kScheme0: return launch_march_k<Pol, K, F | kScheme0>(a, s);
+        case kScheme1: return launch_march_k<Pol, K, F | kScheme1>(a, s);
+        case kScheme2: return launch_march_k<Pol, K, F | kScheme2>(a, s);
+        default: return launch_march_k<Pol, K, F>(a, s);
+    }
+}
+
 }  // namespace
 
 cudaError_t CFS_MARCH_FN(const StageArgs& a, int v, cudaStream_t s) {
     using P = CFS_MARCH_POL;
     constexpr int F = CFS_MARCH_FEAT;
     static_assert(kNumVariants == 13, "variant table and dispatch disagree");
+    constexpr int kDefault = P::kMixed ? kDefaultVariantF32 : kDefaultVariantF64;
+    if (v == kDefault) return launch_march_default<P, kDefault - 1, F>(a, s);
     switch (v) {
         case 1: return launch_march_k<P, 0, F>(a, s);
         case 2: return launch_march_k<P, 1, F>(a, s);
