@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(TI * TJ) stage_kernel(const StageArgs a) {
                 rv = -double(sFX[v][ti + 1][tj] - sFX[v][ti][tj]) / a.dx - double(sFY[v][ti][tj + 1] - sFY[v][ti][tj]) / a.dy;
             }
             if (a.rv && v >= 1)
-                rv += double(static_cast<const T*>(a.rv)[static_cast<long long>(v - 1) * L.nx * L.ny + static_cast<long long>(i) * L.ny + j]);
+                rv += double(static_cast<const T*>(a.rv)[Layout::at(static_cast<long long>(i) * L.ny + j, v - 1)]);
             const double cur = double(sU[v][ti + kGhost][tj + kGhost]);
             double val = cur;
             if (fluid) {
@@ -681,213 +681,6 @@ __global__ void __launch_bounds__(TI * TJ) stage_kernel(const StageArgs a) {
     if (a.P && a.last_stage && a.P->use_cfl) {
         const double m = block_max<NT>(wloc, red);
         if (t == 0 && m > 0.0) atomicMax(&a.P->wmax[1 - a.parity], static_cast<unsigned long long>(__double_as_longlong(m)));
-    }
-}
-
-// --------------------------------------------------- viscous (NS) terms
-// No reference counterpart is live: the reference computes a viscous flux but
-// never adds it (Cell.cpp:128-133, Run.cpp:177,188).  Here: u, v and
-// T = gamma Ma^2 p / rho on the tile and its 3-cell halo (corners included);
-// cell-centred 4th-order derivatives with the reference's table theta_c
-// (FourthOrderCS.h:34-36); at each face the normal derivative from theta_r[1]
-// over 6 cells (FourthOrderCS.h:28-32), the cross derivative and u, v
-// interpolated with zeta_r[1] (FourthOrderCS.h:38-42); stresses
-// sigma_11 = mu (4/3 u_x - 2/3 v_y), sigma_12 = mu (u_y + v_x), heat flux
-// kT T_x with kT = mu / ((gamma-1) Ma^2 Pr).
-// (Functions of a constant table rather than __constant__ arrays: with the
-// loops unrolled every coefficient becomes an immediate, where an array read
-// costs a constant-bank load and, in FP32, a conversion per use.)
-__device__ __forceinline__ double theta_r1(int k) {
-    constexpr double t[6] = {-3.0 / 640, 25.0 / 384, -75.0 / 64, 75.0 / 64, -25.0 / 384, 3.0 / 640};
-    return t[k];
-}
-__device__ __forceinline__ double theta_c(int m) {
-    constexpr double t[5] = {1.0 / 12, -8.0 / 12, 0.0, 8.0 / 12, -1.0 / 12};
-    return t[m];
-}
-__device__ __forceinline__ double zeta1(int k) {
-    constexpr double t[4] = {-1.0 / 16, 9.0 / 16, 9.0 / 16, -1.0 / 16};
-    return t[k];
-}
-
-template <class Pol, int TI, int TJ>
-__global__ void __launch_bounds__(TI * TJ) viscous_kernel(const ViscArgs a) {
-    using T = typename Pol::T;
-    using C = typename Pol::C;
-    constexpr int HI = TI + 2 * kGhost, HJ = TJ + 2 * kGhost;
-    __shared__ C sP[3][HI][HJ];
-    __shared__ C sGY[3][TI + 4][TJ];
-    __shared__ C sGX[3][TI][TJ + 4];
-    __shared__ C sFV[3][TI + 1][TJ];
-    __shared__ C sGV[3][TI][TJ + 1];
-    const Layout& L = a.L;
-    const int i0 = blockIdx.y * TI, j0 = blockIdx.x * TJ;
-    const T* in = static_cast<const T*>(a.in);
-    const int t = threadIdx.x;
-    constexpr bool kF = sizeof(C) == 4;  // FP32 form: constants rounded on the host
-    const C gm1 = kF ? C(a.gm1_f) : C(a.gamma - 1), cT = kF ? C(a.cT_f) : C(a.gamma * a.mach2);
-    // threads as a TI x TJ grid (TJ = 32: one warp per row).  Phases walk rows
-    // by warp and columns by lane.  Items past column TJ (TJ + 4 x-derivatives
-    // and TJ + 1 y-normal faces per row) go to one short extra pass whose lanes
-    // lie whole tile rows apart (distinct shared-memory banks); x-derivatives
-    // and x-normal faces take two rows per thread; the halo tile (TJ + 6 per
-    // row, stored only) numbers its cells row by row over all threads.  So no
-    // warp makes a second pass for a few items.
-    static_assert(TJ == 32, "one warp per tile row");
-    constexpr int NT = TI * TJ;
-    const int ty = t / TJ, tx = t - ty * TJ;
-    for (int e = t; e < HI * HJ; e += NT) {
-        const int r = e / HJ, c = e - r * HJ;
-        const int i = i0 - kGhost + r, j = j0 - kGhost + c;
-        C u = C(0), v = C(0), Tt = C(0);
-        if (i < L.nx + kGhost && j < L.ny + kGhost) {
-            T cv[kVars];
-            ld_cell<T>(in, L.offset(i, j), cv);
-            const C rho = decc<T, C>(cv[0], L, 0), mx = decc<T, C>(cv[1], L, 1);
-            const C my = decc<T, C>(cv[2], L, 2), E = decc<T, C>(cv[3], L, 3);
-            const C rinv = rcp_fast(rho);
-            u = mx * rinv;
-            v = my * rinv;
-            const C p = gm1 * (E - C(0.5) * (mx * mx + my * my) * rinv);
-            Tt = cT * p * rinv;
-        }
-        sP[0][r][c] = u;
-        sP[1][r][c] = v;
-        sP[2][r][c] = Tt;
-    }
-    __syncthreads();
-    const C idx = kF ? C(a.inv_dx_f) : C(a.inv_dx), idy = kF ? C(a.inv_dy_f) : C(a.inv_dy);
-    for (int rr = ty; rr < TI + 4; rr += TI) {  // y-derivatives of rows i0-2 .. i0+TI+1
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            C s = C(0);
-#pragma unroll
-            for (int m = 0; m < 5; ++m) s += C(theta_c(m)) * sP[q][rr + 1][tx + 1 + m];
-            sGY[q][rr][tx] = s * idy;
-        }
-    }
-    // x-derivatives of columns j0-2 .. j0+TJ+1, rows rr and rr+1 per thread
-    // (four of their five stencil values shared): columns 0..TJ-1 by lane,
-    // the 4 past them in a tail whose lanes lie two tile rows apart; on the
-    // top warps, as the y-derivatives' second pass runs on the bottom ones
-    static_assert(TI % 2 == 0, "row pairs");
-    {
-        constexpr int kMain = (TI / 2) * TJ, kCount = kMain + 4 * (TI / 2);
-        constexpr int kFirst = NT - (kCount + 31) / 32 * 32;
-        static_assert(kFirst >= 0, "x-derivative pairs fit in one pass");
-        const int u = t - kFirst;
-        if (u >= 0 && u < kCount) {
-            const int pr = u < kMain ? u / TJ : (u - kMain) % (TI / 2);
-            const int cc = u < kMain ? u % TJ : TJ + (u - kMain) / (TI / 2);
-            const int rr = 2 * pr;
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                C col[6];
-#pragma unroll
-                for (int m = 0; m < 6; ++m) col[m] = sP[q][rr + 1 + m][cc + 1];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    C s = C(0);
-#pragma unroll
-                    for (int m = 0; m < 5; ++m) s += C(theta_c(m)) * col[h + m];
-                    sGX[q][rr + h][cc] = s * idx;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    const C mu = kF ? C(a.mu_f) : C(a.mu), kT = kF ? C(a.kT_f) : C(a.kT), c43 = C(4.0 / 3.0), c23 = C(2.0 / 3.0);
-    // x-normal faces between rows i0+fi-1 and i0+fi, faces fi0 and fi0+1 of a
-    // column per thread (five of their six stencil values shared; TI + 1
-    // faces per column, so the last pair has one face); on the top warps, as
-    // the y-normal faces' tail runs on the bottom one
-    {
-        constexpr int kCount = (TI + 2) / 2 * TJ;
-        constexpr int kFirst = NT - kCount;
-        static_assert(kFirst >= 0, "x-face pairs fit in one pass");
-        const int u = t - kFirst;
-        if (u >= 0) {
-            const int fi0 = 2 * (u / TJ), fj = u % TJ;
-            const bool two = fi0 + 1 <= TI;
-            C dn[2][3], cr[2][3], uf[2] = {C(0), C(0)}, vf[2] = {C(0), C(0)};
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                C col[7], gy[5];
-#pragma unroll
-                for (int k = 0; k < 6; ++k) col[k] = sP[q][fi0 + k][fj + kGhost];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) gy[k] = sGY[q][fi0 + k][fj];
-                col[6] = C(0);
-                gy[4] = C(0);
-                if (two) {
-                    col[6] = sP[q][fi0 + 6][fj + kGhost];
-                    gy[4] = sGY[q][fi0 + 4][fj];
-                }
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    C s = C(0), x = C(0);
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) s += C(theta_r1(k)) * col[h + k];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) x += C(zeta1(k)) * gy[h + k];
-                    dn[h][q] = s * idx;
-                    cr[h][q] = x;
-                    if (q < 2) {
-                        C w = C(0);
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) w += C(zeta1(k)) * col[h + 1 + k];
-                        if (q == 0) uf[h] = w;
-                        else vf[h] = w;
-                    }
-                }
-            }
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (h == 1 && !two) break;
-                const int fi = fi0 + h;
-                const C s11 = mu * (c43 * dn[h][0] - c23 * cr[h][1]);
-                const C s12 = mu * (cr[h][0] + dn[h][1]);
-                sFV[0][fi][fj] = s11;
-                sFV[1][fi][fj] = s12;
-                sFV[2][fi][fj] = uf[h] * s11 + vf[h] * s12 + kT * dn[h][2];
-            }
-        }
-    }
-    for (int pass = 0; pass < 2; ++pass) {  // y-normal faces between columns j0+fj-1 and j0+fj
-        if (pass == 1 && t >= TI) break;
-        const int fi = pass == 0 ? ty : t, fj = pass == 0 ? tx : TJ;
-        C dn[3], cr[3];
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            C s = C(0), x = C(0);
-#pragma unroll
-            for (int k = 0; k < 6; ++k) s += C(theta_r1(k)) * sP[q][fi + kGhost][fj + k];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) x += C(zeta1(k)) * sGX[q][fi][fj + k];
-            dn[q] = s * idy;
-            cr[q] = x;
-        }
-        C uf = C(0), vf = C(0);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            uf += C(zeta1(k)) * sP[0][fi + kGhost][fj + 1 + k];
-            vf += C(zeta1(k)) * sP[1][fi + kGhost][fj + 1 + k];
-        }
-        const C s22 = mu * (c43 * dn[1] - c23 * cr[0]);
-        const C s21 = mu * (dn[0] + cr[1]);
-        sGV[0][fi][fj] = s21;
-        sGV[1][fi][fj] = s22;
-        sGV[2][fi][fj] = uf * s21 + vf * s22 + kT * dn[2];
-    }
-    __syncthreads();
-    const int ti = t / TJ, tj = t - (t / TJ) * TJ;
-    const int i = i0 + ti, j = j0 + tj;
-    if (i < L.nx && j < L.ny) {
-        T* rv = static_cast<T*>(a.rv);
-        const long long n = static_cast<long long>(L.nx) * L.ny, k = static_cast<long long>(i) * L.ny + j;
-#pragma unroll
-        for (int q = 0; q < 3; ++q)
-            rv[q * n + k] = T((sFV[q][ti + 1][tj] - sFV[q][ti][tj]) * idx + (sGV[q][ti][tj + 1] - sGV[q][ti][tj]) * idy);
     }
 }
 

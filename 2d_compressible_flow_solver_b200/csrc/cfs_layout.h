@@ -95,7 +95,7 @@ struct StageArgs {
     int parity;            // graph mode: which wmax slot holds this step's max
     int last_stage;        // 1: accumulate the CFL max of the new state into P->wmax[1-parity]
     int first_stage;       // 1: reset P->wmax[1-parity], advance P->t
-    const void* rv;        // optional viscous RHS (rho u, rho v, E) [3][nx][ny], storage type
+    const void* rv;        // optional viscous RHS (rho u, rho v, E, unused) [nx][ny][4], storage type
     int variant;           // throughput-form kernel variant (1-based; 0 = default)
     int positivity;        // 0 off, 1 face-state fallback, 2 also first order near the body, 3 also floors
     const uint8_t* lowo;   // positivity 2: [nx+1][ny+1] face flags, bit 0 x-face (i-1/2, j),
@@ -185,7 +185,7 @@ CFS_HD int march_features(const StageArgs& a) {
 }
 
 // Viscous (Navier-Stokes) RHS of one state: (dFv/dx + dGv/dy) for the momentum
-// and energy equations, written to rv[3][nx][ny].
+// and energy equations, written to rv[nx][ny][4] (the fourth word 0).
 struct ViscArgs {
     const void* in;
     void* rv;
@@ -195,6 +195,7 @@ struct ViscArgs {
     // the FP32 form's constants, rounded once on the host: gamma - 1,
     // gamma Ma^2, mu, kT, 1/dx, 1/dy
     float gm1_f, cT_f, mu_f, kT_f, inv_dx_f, inv_dy_f;
+    int rows;               // rows of a warp's work item (set by the launcher)
 };
 
 struct IbArgs {

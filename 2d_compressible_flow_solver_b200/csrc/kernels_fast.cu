@@ -1,10 +1,12 @@
 // Kernels of the throughput forms: FP64 with FMA contraction and the
 // FP32-mixed form.  Built with FMA contraction on (nvcc default).
 #include <atomic>
+#include <mutex>
 
 #include "cfs_kernels.cuh"
 #include "cfs_launch.h"
 #include "cfs_march.cuh"
+#include "cfs_viscous.cuh"
 
 namespace cfs {
 
@@ -19,9 +21,10 @@ cudaError_t launch_boundary_flux(const StageArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+constexpr int kMaxDev = 64;
+
 // SM count of the current device (cached per device).
 int sm_count() {
-    constexpr int kMaxDev = 64;
     static std::atomic<int> count[kMaxDev] = {};  // every writer stores the same value
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return 148;
@@ -174,26 +177,41 @@ int batch_blocks_per_sm(Prec p) {
     return n > 0 ? n : 1;
 }
 
-constexpr int kViscTI = 8;
-constexpr int kViscTJ = 32;
-// FP32 tiles twice as tall: the 3-cell halo of the primitive, gradient and
-// face phases is recomputed on fewer cells (37.5 KB of static shared memory;
-// the FP64 tile would not fit in 48 KB)
-constexpr int kViscTI32 = 16;
-
-inline dim3 visc_grid(const Layout& L, int ti) {
-    return dim3((L.ny + kViscTJ - 1) / kViscTJ, (L.nx + ti - 1) / ti);
-}
-
-cudaError_t launch_viscous_f64(const ViscArgs& a, cudaStream_t s) {
-    viscous_kernel<PolF64, kViscTI, kViscTJ><<<visc_grid(a.L, kViscTI), kViscTI * kViscTJ, 0, s>>>(a);
+// Rows of a viscous work item by the row march's rule: an item of R rows
+// costs about R + 2.5 (five more rows are loaded and converted, one more
+// x-face formed).
+template <class Pol, int kMinBlocks>
+cudaError_t launch_viscous_form(const ViscArgs& a_in, cudaStream_t s) {
+    static std::once_flag once[kMaxDev];
+    static long long slots_of[kMaxDev];
+    auto query = []() -> long long {
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, viscous_kernel<Pol, kMinBlocks>, 32 * kViscWarps, 0) != cudaSuccess) {
+            (void)cudaGetLastError();  // a failed query leaves no error behind
+            return 0;
+        }
+        return static_cast<long long>(per_sm) * sm_count();
+    };
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    long long slots = 0;
+    if (dev < 0 || dev >= kMaxDev) {
+        slots = query();
+    } else {
+        std::call_once(once[dev], [&] { slots_of[dev] = query(); });
+        slots = slots_of[dev];
+    }
+    ViscArgs a = a_in;
+    const int nseg = (a.L.ny + kViscSeg - 1) / kViscSeg;
+    a.rows = slots > 0 ? choose_rows(nseg, kViscWarps, a.L.nx, slots) : 32;
+    const long long items = static_cast<long long>(nseg) * ((a.L.nx + a.rows - 1) / a.rows);
+    viscous_kernel<Pol, kMinBlocks><<<static_cast<unsigned>((items + kViscWarps - 1) / kViscWarps), 32 * kViscWarps, 0, s>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t launch_viscous_f32(const ViscArgs& a, cudaStream_t s) {
-    viscous_kernel<PolF32, kViscTI32, kViscTJ><<<visc_grid(a.L, kViscTI32), kViscTI32 * kViscTJ, 0, s>>>(a);
-    return cudaGetLastError();
-}
+cudaError_t launch_viscous_f64(const ViscArgs& a, cudaStream_t s) { return launch_viscous_form<PolF64, 3>(a, s); }
+cudaError_t launch_viscous_f32(const ViscArgs& a, cudaStream_t s) { return launch_viscous_form<PolF32, 5>(a, s); }
 
 cudaError_t launch_weno_faces_f64(int n, const double* st, double* l, double* r, double g, double eps, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
