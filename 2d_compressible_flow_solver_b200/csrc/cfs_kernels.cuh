@@ -11,6 +11,33 @@
 
 namespace cfs {
 
+// ------------------------------------------------ dependent launches
+// The kernels of a stage are launched as programmatic dependents of the kernel
+// before them in the stream (launch_after): their blocks are brought onto the
+// SMs, and find their work item, while that kernel still runs, and then wait
+// for its end (after_previous, before the first access to memory that a
+// kernel writes).  Every kernel lets its own dependents in at once
+// (let_next_in); they wait in turn, so the order of the stages is that of
+// plain launches.  SSP3 steps of the 605 x 301 cylinder in FP64 (three kernels
+// a stage) 82.8 -> 78.8 us, of the 2048 x 1024 one in FP32 259 -> 256.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void let_next_in() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
+template <class... Params, class... Args>
+inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t dyn, cudaStream_t s, Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = dyn;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // ---------------------------------------------------------------- policies
 // T = storage type of the state, C = type of the WENO/HLL arithmetic.
 struct PolExact { using T = double; using C = double; static constexpr bool kExact = true;  static constexpr bool kMixed = false; };
@@ -23,6 +50,13 @@ enum { kHllReference = 0, kHllDavis = 1 };
 // Reconstructed face state: conserved variables, pressure, sound speed and
 // (throughput forms) 1/rho.
 template <class C> struct Face5 { C r, mx, my, E, p, a, ri; };
+
+// A product that is rounded by itself.  The throughput forms write every
+// multiply-add as fma() and every product that enters a sum otherwise as
+// mul(), so no contraction is left to the compiler and a cell's result is the
+// same bits in every kernel that computes it (row march, tile form, batch).
+__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 
 // FP32 reciprocal and reciprocal square root of the throughput forms: the
 // PTX approximations themselves (one MUFU instruction each, maximum error
@@ -75,7 +109,7 @@ __device__ __forceinline__ double sqrt_pos(double x) {
     return fma(0.5 * y, fma(-sq, sq, x), sq);
 }
 __device__ __forceinline__ float rcp_pos(float x) { return rcp_fast(x); }
-__device__ __forceinline__ float sqrt_fast(float x) { return x * rsqrt_fast(x); }
+__device__ __forceinline__ float sqrt_fast(float x) { return mul(x, rsqrt_fast(x)); }
 __device__ __forceinline__ double sqrt_fast(double x) { return sqrt(x); }
 
 // One cell's four stored variables in vector accesses (one 16-byte access in
@@ -221,21 +255,21 @@ __device__ __forceinline__ void finish_state(Face5<typename Pol::C>& s, double g
     } else if constexpr (Pol::kMixed) {
         const C rinv = rcp_fast(s.r);
         s.ri = rinv;
-        const C ke = C(0.5) * (s.mx * s.mx + s.my * s.my) * rinv;
-        if (ke > C(0.9) * s.E) {
+        const C t = fma(C(-0.5), mul(fma(s.mx, s.mx, mul(s.my, s.my)), rinv), s.E);  // E - ke
+        if (t < C(0.1) * s.E) {
             const double r = s.r, mx = s.mx, my = s.my, E = s.E;
-            const double p = (g - 1) * (E - 0.5 * (mx * mx + my * my) / r);
+            const double p = (g - 1) * (E - 0.5 * fma(mx, mx, mul(my, my)) / r);
             s.p = C(p);
             s.a = C(sqrt(g * p / r));
         } else {
-            s.p = C(g - 1) * (s.E - ke);
-            s.a = sqrt_fast(C(g) * s.p * rinv);
+            s.p = mul(C(g - 1), t);
+            s.a = sqrt_fast(mul(mul(C(g) * C(g - 1), t), rinv));
         }
     } else {
         const C rinv = rcp_pos(s.r);
         s.ri = rinv;
-        s.p = C(g - 1) * (s.E - C(0.5) * (s.mx * s.mx + s.my * s.my) * rinv);
-        s.a = sqrt_pos(C(g) * s.p * rinv);
+        s.p = mul(C(g - 1), fma(C(-0.5) * fma(s.mx, s.mx, mul(s.my, s.my)), rinv, s.E));
+        s.a = sqrt_pos(mul(mul(C(g), s.p), rinv));
     }
 }
 
@@ -258,11 +292,11 @@ __device__ __forceinline__ void phys_flux(const Face5<typename Pol::C>& s, int d
         }
     } else {
         const C q = dir == 0 ? s.mx : s.my;
-        const C un = q * s.ri;
+        const C un = mul(q, s.ri);
         F[0] = q;
-        F[1] = s.mx * un + (dir == 0 ? s.p : C(0));
-        F[2] = s.my * un + (dir == 0 ? C(0) : s.p);
-        F[3] = (s.E + s.p) * un;
+        F[1] = dir == 0 ? fma(s.mx, un, s.p) : mul(s.mx, un);
+        F[2] = dir == 0 ? mul(s.my, un) : fma(s.my, un, s.p);
+        F[3] = mul(s.E + s.p, un);
     }
 }
 
@@ -299,20 +333,20 @@ __device__ __forceinline__ void hll_flux(const Face5<typename Pol::C>& L, const 
             SR = max_ref(uL + aL, uR + aR);
         }
     } else {
-        const C uL = qL * L.ri, uR = qR * R.ri;
+        const C uL = mul(qL, L.ri), uR = mul(qR, R.ri);
         if (variant == kHllReference) {
             const C a_ave = C(0.5) * (aL + aR);
             const C rho_ave = C(0.5) * (L.r + R.r);
-            const C ra = rho_ave * a_ave;
+            const C ra = mul(rho_ave, a_ave);
             const C inv_ra = rcp_pos(ra);  // ra > 0: mean density times mean sound speed
-            const C p_star = C(0.5) * (L.p + R.p) - C(0.5) * (uR - uL) * ra;
-            const C u_star = C(0.5) * (uR + uL) - C(0.5) * (R.p - L.p) * inv_ra;
-            const C ratio = rho_ave * rho_ave * inv_ra;
-            const C rho_star_L = L.r + (uL - u_star) * ratio;
-            const C rho_star_R = R.r - (uR - u_star) * ratio;
-            const C gp = C(g) * p_star;
-            const C a_star_L = sqrt_fast(gp * rcp_fast(rho_star_L));
-            const C a_star_R = sqrt_fast(gp * rcp_fast(rho_star_R));
+            const C p_star = fma(C(-0.5) * (uR - uL), ra, C(0.5) * (L.p + R.p));
+            const C u_star = fma(C(-0.5) * (R.p - L.p), inv_ra, C(0.5) * (uR + uL));
+            const C ratio = mul(mul(rho_ave, rho_ave), inv_ra);
+            const C rho_star_L = fma(uL - u_star, ratio, L.r);
+            const C rho_star_R = fma(u_star - uR, ratio, R.r);
+            const C gp = mul(C(g), p_star);
+            const C a_star_L = sqrt_fast(mul(gp, rcp_fast(rho_star_L)));
+            const C a_star_R = sqrt_fast(mul(gp, rcp_fast(rho_star_R)));
             SL = min_ref(qL - aL, u_star - a_star_L);
             SR = max_ref(qL + aL, u_star + a_star_R);
         } else {
@@ -399,6 +433,15 @@ __device__ __forceinline__ double rk_update(int rk, int stage, double dt, double
     return (1.0 / 3.0) * u0v + (2.0 / 3.0) * cur + (2.0 / 3.0) * dt * r;
 }
 
+// The FP64 throughput form's update: the same coefficients (x1: the current
+// state, or U^1 in the last stage of TVD3 as written), fused multiply-adds.
+__device__ __forceinline__ double rk_update_fast(int rk, int stage, double dt, double u0v, double x1, double r) {
+    if (stage == 0) return fma(dt, r, x1);
+    if (rk == kRkTvd2) return fma(0.5 * dt, r, fma(0.5, u0v, 0.5 * x1));
+    if (stage == 1) return fma(0.25 * dt, r, fma(0.75, u0v, 0.25 * x1));
+    return fma(mul(2.0 / 3.0, dt), r, fma(1.0 / 3.0, u0v, mul(2.0 / 3.0, x1)));
+}
+
 // ------------------------------------------------------ stochastic rounding
 // FP32 storage of the FP32-mixed form rounds each new state value
 // stochastically (no reference counterpart): to one of the two floats around
@@ -459,7 +502,7 @@ __device__ __forceinline__ void floor_state(double s[kVars], double g) {
         mx = my = 0.0;
         E = kPFloor / (g - 1);
     }
-    const double ke = 0.5 * (mx * mx + my * my) / rho;
+    const double ke = 0.5 * fma(mx, mx, mul(my, my)) / rho;
     if (!((g - 1) * (E - ke) > kPFloor)) E = kPFloor / (g - 1) + ke;
     s[0] = rho;
     s[1] = mx;
@@ -491,10 +534,10 @@ __device__ __forceinline__ double cfl_term(double w) {
 template <class C>
 __device__ __forceinline__ C wave_sum_fast(C rho, C mx, C my, C E, C g, C inv_dx, C inv_dy) {
     const C ri = rcp_fast(rho);
-    const C u = mx * ri, v = my * ri;
-    const C p = (g - C(1)) * (E - C(0.5) * (mx * u + my * v));
-    const C a = sqrt_fast(g * p * ri);
-    return (fabs(u) + a) * inv_dx + (fabs(v) + a) * inv_dy;
+    const C u = mul(mx, ri), v = mul(my, ri);
+    const C p = mul(g - C(1), fma(C(-0.5), fma(mx, u, mul(my, v)), E));
+    const C a = sqrt_fast(mul(mul(g, p), ri));
+    return fma(fabs(u) + a, inv_dx, mul(fabs(v) + a, inv_dy));
 }
 
 // Writes one cell of the new state and the ghost copies it feeds: Neumann
@@ -565,6 +608,8 @@ __global__ void __launch_bounds__(TI * TJ) stage_kernel(const StageArgs a) {
     const int i0 = blockIdx.y * TI, j0 = blockIdx.x * TJ;
     const T* in = static_cast<const T*>(a.in);
     const int t = threadIdx.x;
+    let_next_in();
+    after_previous();
 
     for (int e = t; e < HI * HJ; e += NT) {
         const int r = e / HJ, c = e - r * HJ;
@@ -757,6 +802,8 @@ __device__ __forceinline__ void ib_fill_one(const IbArgs& a, int g) {
 template <class T>
 __global__ void ib_fill_kernel(const IbArgs a) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    let_next_in();
+    after_previous();
     if (g >= a.n) return;
     ib_fill_one<T>(a, g);
 }
@@ -767,6 +814,8 @@ template <class T>
 __global__ void batch_ib_fill_kernel(const IbArgs* __restrict__ args, const int* __restrict__ cases,
                                      const int* __restrict__ local, int total) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    let_next_in();
+    after_previous();
     if (g >= total) return;
     const IbArgs a = args[cases[g]];
     ib_fill_one<T>(a, local[g]);

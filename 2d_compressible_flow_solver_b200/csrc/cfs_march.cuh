@@ -58,7 +58,7 @@ constexpr int kSeg = 30;
 template <class C>
 __device__ __forceinline__ void weno5_pair_diff(C v0, C v1, C v2, C v3, C v4, C eps, C& left, C& right) {
     const C D1 = v1 - v0, D2 = v2 - v1, D3 = v3 - v2, D4 = v4 - v3;
-    const C P2 = D2 * D2, P3 = D3 * D3;
+    const C P2 = mul(D2, D2), P3 = mul(D3, D3);
     C q0 = fma(D1, fma(C(-2.75), D2, D1), fma(C(2.5), P2, eps));  // eps: the WENO eps times 3/4
     C q1 = fma(D2, fma(C(-1.25), D3, D2), P3 + eps);
     C q2 = fma(D4, fma(C(-2.75), D3, D4), fma(C(2.5), P3, eps));
@@ -70,19 +70,19 @@ __device__ __forceinline__ void weno5_pair_diff(C v0, C v1, C v2, C v3, C v4, C 
     q0 *= q0;
     q1 *= q1;
     q2 *= q2;
-    const C X = q1 * q2, Y = q0 * q2, Z = q0 * q1;
-    const C X5 = C(5.0 / 12.0) * X, Z5 = C(5.0 / 12.0) * Z;
+    const C X = mul(q1, q2), Y = mul(q0, q2), Z = mul(q0, q1);
+    const C X5 = mul(C(5.0 / 12.0), X), Z5 = mul(C(5.0 / 12.0), Z);
     const C h = fma(C(2), Y, X + Z);
     const C A0 = fma(C(-0.4), D1, D2), A1 = fma(C(0.5), D2, D3), A2 = fma(C(-0.25), D4, D3);
     const C B0 = fma(C(-0.4), D4, D3), B1 = fma(C(0.5), D3, D2), B2 = fma(C(-0.25), D1, D2);
     // (the weight sums are >= 5 eps^4 > 0: rcp_pos)
-    left = fma(fma(X5, A0, fma(Y, A1, Z * A2)), rcp_pos(fma(C(1.5), h, -X)), v2);
-    right = fma(fma(Z5, B0, fma(Y, B1, X * B2)), -rcp_pos(fma(C(1.5), h, -Z)), v2);
+    left = fma(fma(X5, A0, fma(Y, A1, mul(Z, A2))), rcp_pos(fma(C(1.5), h, -X)), v2);
+    right = fma(fma(Z5, B0, fma(Y, B1, mul(X, B2))), -rcp_pos(fma(C(1.5), h, -Z)), v2);
 }
 
 template <class C>
 __device__ __forceinline__ void weno5_pair(C v0, C v1, C v2, C v3, C v4, C eps, C& left, C& right) {
-    weno5_pair_diff(v0, v1, v2, v3, v4, C(0.75) * eps, left, right);
+    weno5_pair_diff(v0, v1, v2, v3, v4, mul(C(0.75), eps), left, right);
 }
 
 // The same pair for two variables at once in packed FP32 (sm_100 FFMA2 /
@@ -128,20 +128,19 @@ __device__ __forceinline__ void finish_pair(Face5<typename Pol::C>& L, Face5<typ
     if constexpr (Pol::kMixed) {
         const float gm1 = float(g - 1), gg = float(g) * float(g - 1);
         const float riL = rcp_fast(L.r), riR = rcp_fast(R.r);
-        const float tL = fmaf(-0.5f, fmaf(L.mx, L.mx, L.my * L.my) * riL, L.E);
-        const float tR = fmaf(-0.5f, fmaf(R.mx, R.mx, R.my * R.my) * riR, R.E);
+        const float tL = fmaf(-0.5f, mul(fmaf(L.mx, L.mx, mul(L.my, L.my)), riL), L.E);
+        const float tR = fmaf(-0.5f, mul(fmaf(R.mx, R.mx, mul(R.my, R.my)), riR), R.E);
         if (tL < 0.1f * L.E || tR < 0.1f * R.E) {
             finish_state<Pol>(L, g);
             finish_state<Pol>(R, g);
             return;
         }
-        const float a2L = gg * tL * riL, a2R = gg * tR * riR;
         L.ri = riL;
         R.ri = riR;
-        L.p = gm1 * tL;
-        R.p = gm1 * tR;
-        L.a = a2L * rsqrt_fast(a2L);
-        R.a = a2R * rsqrt_fast(a2R);
+        L.p = mul(gm1, tL);
+        R.p = mul(gm1, tR);
+        L.a = sqrt_fast(mul(mul(gg, tL), riL));
+        R.a = sqrt_fast(mul(mul(gg, tR), riR));
     } else {
         finish_state<Pol>(L, g);
         finish_state<Pol>(R, g);
@@ -461,6 +460,8 @@ template <class Pol>
 __global__ void __launch_bounds__(128) boundary_flux_kernel(const StageArgs a) {
     const int s = blockIdx.y;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    let_next_in();
+    after_previous();
     if (a.bc[s] != kDirichlet || k >= (s < 2 ? a.L.ny : a.L.nx)) return;
     boundary_face_flux<Pol>(a, s, k);
 }
@@ -471,8 +472,251 @@ __global__ void __launch_bounds__(128) batch_boundary_flux_kernel(const StageArg
     const StageArgs& a = args[blockIdx.z];
     const int s = blockIdx.y;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    let_next_in();
+    after_previous();
     if (!a.bflux || a.bc[s] != kDirichlet || k >= (s < 2 ? a.L.ny : a.L.nx)) return;
     boundary_face_flux<Pol>(a, s, k);
+}
+
+// What the update of a stage's cells shares.
+struct UpdateCoefs {
+    double dt, inv_dx, inv_dy;
+    float inv_dxf, inv_dyf;
+    // FP32: new = cA x0 + cB x1 + (c dt) R with x0 = U^0 (or the current state
+    // at stage 0), x1 = U^1 (TVD3 as written, stage 2) or the current state
+    // (TVD2rdRK.h:16-19, TVD3rdRK.h:14-18).  cA + cB must be exactly 1 in FP32,
+    // else the deviation form scales the stored deviations by (cA + cB) every
+    // step: cB = fl(2/3), cA = 1 - cB (an exact FP32 subtraction).
+    float cA, cB, cdt;
+    bool x1_u1, sr;
+    unsigned int step_seed;
+    bool do_cfl;
+};
+
+template <class Pol, int kFeat>
+__device__ __forceinline__ UpdateCoefs update_coefs(const StageArgs& a) {
+    UpdateCoefs k;
+    const double dt = stage_dt(a);
+    k.dt = dt;
+    k.inv_dx = 1.0 / a.dx;
+    k.inv_dy = 1.0 / a.dy;
+    k.inv_dxf = float(k.inv_dx);
+    k.inv_dyf = float(k.inv_dy);
+    k.cA = 1.0f;
+    k.cB = 0.0f;
+    double cdtd = dt;  // dt coefficient of the stage, FP64
+    k.x1_u1 = false;
+    if (a.stage == 1) {
+        if (a.rk == kRkTvd2) { k.cA = 0.5f; k.cB = 0.5f; cdtd = 0.5 * dt; }
+        else { k.cA = 0.75f; k.cB = 0.25f; cdtd = 0.25 * dt; }
+    } else if (a.stage == 2) {
+        k.cB = float(2.0 / 3.0);
+        k.cA = 1.0f - k.cB;
+        cdtd = (2.0 / 3.0) * dt;
+        k.x1_u1 = a.rk == kRkTvd3Ref;
+    }
+    if (kFeat & kSchemeU1) k.x1_u1 = true;
+    if (kFeat & kSchemeNoU1) k.x1_u1 = false;
+    k.cdt = float(cdtd);
+    // Stochastic rounding of the state that ends each step (the last stage), or
+    // of every stage (CFS_ROUND_STOCHASTIC_ALL); otherwise round to nearest.
+    // Rounding an intermediate stage to nearest leaves a small mass bias: its
+    // increments are dt times differences of FP32 fluxes, a coarse lattice on
+    // the stored grid, so the rounding errors do not average out.
+    const bool last_of_step = a.rk == kRkTvd2 ? a.stage == 1 : a.stage == 2;
+    k.sr = Pol::kMixed && ((kFeat & kSchemeSr) || stage_rounds_stochastically(a.rounding, last_of_step));
+    k.step_seed = (a.P ? a.P->seed[a.parity] : a.seed) * 4u + static_cast<unsigned int>(a.stage);
+    k.do_cfl = a.P && a.last_stage && a.P->use_cfl;  // read once: stores to `out` may alias P for the compiler
+    return k;
+}
+
+// Start of a step in graph mode: the next step's CFL slot, the time, the seed
+// (one thread of the grid's first item).
+__device__ __forceinline__ void begin_step(const StageArgs& a, double dt) {
+    a.P->wmax[1 - a.parity] = 0ull;
+    a.P->t += dt;
+    a.P->dt_last = dt;
+    a.P->seed[1 - a.parity] = a.P->seed[a.parity] + 1u;
+}
+
+// Update of cell (i, j) from its x-fluxes FX (upper) and FXp (lower), the y
+// part RY of its RHS and, with kFeatExtra, its viscous RHS rvc; cur, u0, u1:
+// stored values of the current state, U^0 and U^1 (as the stage reads them).
+// Stores the new state and its ghost copies and raises wloc to the cell's
+// CFL term.
+template <class Pol, int kFeat>
+__device__ __forceinline__ void update_cell(const StageArgs& a, const UpdateCoefs& k, int i, int j,
+                                            const typename Pol::C FX[kVars], const typename Pol::C FXp[kVars],
+                                            const typename Pol::C RY[kVars], const typename Pol::T rvc[kVars],
+                                            const typename Pol::T cur[kVars], const typename Pol::T u0[kVars],
+                                            const typename Pol::T u1[kVars], bool fluid, double& wloc) {
+    using T = typename Pol::T;
+    using C = typename Pol::C;
+    constexpr bool kPos = (kFeat & kFeatPos) != 0;
+    constexpr bool kExtra = (kFeat & kFeatExtra) != 0;
+    const Layout& L = a.L;
+    const double g = a.gamma;
+    double* const rhs_out = kExtra ? a.rhs : nullptr;
+    const bool has_rv = kExtra && a.rv;
+    C nv[kVars];  // new state in the form's arithmetic type, for the CFL maximum
+    T sv[kVars];
+    if constexpr (Pol::kMixed) {
+        // FP32 update of the stored deviations (value - off): the RK
+        // coefficients of a stage sum to 1, so the offsets cancel and
+        // the rounding step is that of the deviation.
+        // (formed for every cell and selected: a non-fluid cell keeps its state)
+        float rvf[kVars], x1[kVars], ndv[kVars];
+#pragma unroll
+        for (int v = 0; v < kVars; ++v) {
+            rvf[v] = fmaf(-(FX[v] - FXp[v]), k.inv_dxf, RY[v]);
+            if (has_rv && v >= 1) rvf[v] += rvc[v - 1];
+            // (stage 0: cB = 0 and x1 - x0 = 0, so x1 adds nothing)
+            x1[v] = k.x1_u1 ? u1[v] : cur[v];
+        }
+        if (k.sr) {
+            // Stochastic rounding of x0 + cB (x1 - x0) + cdt R (cA = 1 - cB
+            // exactly): the increment is formed first, at its own
+            // spacing (roundings near 1e-12 of the state, far below the
+            // stored spacing), gets a dither uniform over one stored
+            // spacing of the result's binade, and is added to x0 with
+            // one rounding; two variables per packed instruction.
+            const unsigned int h = cell_hash(i, j, k.step_seed);
+            const float u[kVars] = {dither_bits<0>(h), dither_bits<1>(h), dither_bits<2>(h), dither_bits<3>(h)};
+#pragma unroll
+            for (int v = 0; v < kVars; v += 2) {
+                const float2 a0 = make_float2(u0[v], u0[v + 1]);
+                const float2 inc = fma2(p2(k.cB), sub2(make_float2(x1[v], x1[v + 1]), a0),
+                                        mul2(p2(k.cdt), make_float2(rvf[v], rvf[v + 1])));
+                const float2 f = add2(a0, inc);
+                const float2 t = add2(make_float2(u[v], u[v + 1]), p2(-kDitherCentre));
+                const float2 r = add2(a0, fma2(make_float2(binade(f.x), binade(f.y)), t, inc));
+                ndv[v] = r.x;
+                ndv[v + 1] = r.y;
+            }
+        } else {
+#pragma unroll
+            for (int v = 0; v < kVars; ++v) ndv[v] = fmaf(k.cdt, rvf[v], fmaf(k.cA, u0[v], mul(k.cB, x1[v])));
+        }
+#pragma unroll
+        for (int v = 0; v < kVars; ++v) {
+            const float nd = fluid ? ndv[v] : cur[v];
+            sv[v] = nd;
+            nv[v] = nd + L.off[v];
+            if (kExtra && rhs_out)
+                rhs_out[static_cast<long long>(v) * L.nx * L.ny + static_cast<long long>(i) * L.ny + j] = fluid ? double(rvf[v]) : 0.0;
+        }
+    } else {
+#pragma unroll
+        for (int v = 0; v < kVars; ++v) {
+            double rv = fma(-(FX[v] - FXp[v]), k.inv_dx, RY[v]);
+            if (has_rv && v >= 1) rv += rvc[v - 1];
+            const double val = fluid ? rk_update_fast(a.rk, a.stage, k.dt, u0[v], k.x1_u1 ? u1[v] : cur[v], rv) : cur[v];
+            sv[v] = val;
+            nv[v] = val;
+            if (kExtra && rhs_out)
+                rhs_out[static_cast<long long>(v) * L.nx * L.ny + static_cast<long long>(i) * L.ny + j] = fluid ? rv : 0.0;
+        }
+    }
+    if (kPos && a.positivity >= kPosFloor && fluid) {
+        // p > floor, multiplied by rho > 0: (g-1)(rho E - |m|^2/2) > floor rho
+        const C q = fma(nv[3], nv[0], C(-0.5) * fma(nv[1], nv[1], mul(nv[2], nv[2])));
+        if (!(nv[0] > C(kRhoFloor)) || !(C(g - 1.0) * q > C(kPFloor) * nv[0])) {
+            double s[kVars];
+#pragma unroll
+            for (int v = 0; v < kVars; ++v)
+                s[v] = Pol::kMixed ? double(sv[v]) + double(L.off[v]) : double(nv[v]);
+            floor_state(s, g);
+#pragma unroll
+            for (int v = 0; v < kVars; ++v) {
+                sv[v] = Pol::kMixed ? T(s[v] - double(L.off[v])) : T(s[v]);
+                nv[v] = C(s[v]);
+            }
+        }
+    }
+    store_cell4<T>(static_cast<T*>(a.out), L, a.bc, i, j, sv);
+    if (k.do_cfl) {
+        const double w = cfl_term(double(wave_sum_fast<C>(nv[0], nv[1], nv[2], nv[3], C(g), C(k.inv_dx), C(k.inv_dy))));
+        if (fluid && w > wloc) wloc = w;
+    }
+}
+
+// The CFL maximum of a warp's cells: one atomic per warp (no block barrier, so
+// the warps of a block never wait for each other).
+__device__ __forceinline__ void raise_wmax(const StageArgs& a, double wloc) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) wloc = fmax(wloc, __shfl_xor_sync(0xffffffffu, wloc, o));
+    if ((threadIdx.x & 31) == 0 && wloc > 0.0)
+        atomicMax(&a.P->wmax[1 - a.parity], static_cast<unsigned long long>(__double_as_longlong(wloc)));
+}
+
+// Flux through the x-face below row r in the column j where that face is a
+// physical one (r = 0 or nx): the cell's own (transmissive; c: the interior
+// cell's values) or the precomputed one (Dirichlet).
+template <class Pol>
+__device__ __forceinline__ void boundary_x_flux(const StageArgs& a, int r, int j, const typename Pol::C c[kVars],
+                                                typename Pol::C FX[kVars]) {
+    const Layout& L = a.L;
+    // (no side index computed at run time: it would put the batch's argument block into local memory)
+    if (r == 0 ? a.bc[0] == kNeumann : a.bc[1] == kNeumann) {
+        wall_flux<Pol>(c, 0, a.gamma, FX);
+    } else if (j >= 0 && j < L.ny) {
+        const typename Pol::C* b = static_cast<const typename Pol::C*>(a.bflux) + bflux_side_offset(L, r == 0 ? 0 : 1);
+#pragma unroll
+        for (int v = 0; v < kVars; ++v) FX[v] = b[static_cast<long long>(v) * L.ny + j];
+    }
+}
+
+// The y part of row r's RHS, RY, for the lanes of a warp on consecutive
+// columns j (the warp's first lane on the segment's first column less one): WENO
+// states of the 5-cell stencils st, the flux above each lane's cell, the
+// difference of the two.  The outer lanes' RY are not those of their cells.
+template <class Pol, int kFeat, bool kDeviations>
+__device__ __forceinline__ void y_part(const StageArgs& a, const UpdateCoefs& k, int r, int j, int hll,
+                                       const typename Pol::C st[5][kVars], typename Pol::C eps, unsigned int f_r,
+                                       bool warp_ybnd, bool ybnd, const typename Pol::C* bfy, typename Pol::C RY[kVars]) {
+    using C = typename Pol::C;
+    const Layout& L = a.L;
+    const double g = a.gamma;
+    auto full = [&](const C w[kVars], C out[kVars]) {
+#pragma unroll
+        for (int v = 0; v < kVars; ++v) out[v] = kDeviations ? w[v] + C(L.off[v]) : w[v];
+    };
+    Face5<C> Ly, Ry;
+    cell_states<Pol>(st, eps, g, Ly, Ry, kDeviations ? L.off : nullptr);
+    if constexpr ((kFeat & kFeatPos) != 0) {
+        C cc[kVars];
+        full(st[2], cc);
+        fix_states<Pol>(f_r & kCellLowYhi, f_r & kCellLowYlo, cc, g, Ly, Ry);
+    }
+    // right state of the cell above (lane + 1)
+    Face5<C> Rn;
+    Rn.r = __shfl_down_sync(0xffffffffu, Ry.r, 1);
+    Rn.mx = __shfl_down_sync(0xffffffffu, Ry.mx, 1);
+    Rn.my = __shfl_down_sync(0xffffffffu, Ry.my, 1);
+    Rn.E = __shfl_down_sync(0xffffffffu, Ry.E, 1);
+    Rn.p = __shfl_down_sync(0xffffffffu, Ry.p, 1);
+    Rn.a = __shfl_down_sync(0xffffffffu, Ry.a, 1);
+    Rn.ri = __shfl_down_sync(0xffffffffu, Ry.ri, 1);
+    // face between column j and j+1 (face index j+1)
+    C FY[kVars];
+    hll_flux<Pol>(Ly, Rn, 1, hll, g, FY);
+    if (warp_ybnd && ybnd) {
+        if (bfy) {
+#pragma unroll
+            for (int v = 0; v < kVars; ++v) FY[v] = bfy[static_cast<long long>(v) * L.nx + r];
+        } else {  // the interior cell: column 0 for the lane below it, this lane's at the top
+            C c[kVars];
+#pragma unroll
+            for (int v = 0; v < kVars; ++v) c[v] = j == -1 ? st[3][v] : st[2][v];
+            full(c, c);
+            wall_flux<Pol>(c, 1, g, FY);
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < kVars; ++v) {
+        const C below = __shfl_up_sync(0xffffffffu, FY[v], 1);
+        RY[v] = mul(below - FY[v], Pol::kMixed ? C(k.inv_dyf) : C(k.inv_dy));
+    }
 }
 
 // One work item: rows [by*rows, by*rows + rows) of segment `seg` (columns
@@ -526,53 +770,15 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
     const T* in = static_cast<const T*>(a.in);
     const C eps = C(a.eps);
     const double g = a.gamma;
-    const double dt = stage_dt(a);
-    const double inv_dx = 1.0 / a.dx, inv_dy = 1.0 / a.dy;
-    const float inv_dxf = float(inv_dx), inv_dyf = float(inv_dy);
-    // FP32 update coefficients of this stage: new = cA x0 + cB x1 + (c dt) R with
-    // x0 = U^0 (or the current state at stage 0), x1 = U^1 (TVD3 as written,
-    // stage 2) or the current state (TVD2rdRK.h:16-19, TVD3rdRK.h:14-18).
-    float cA = 1.0f, cB = 0.0f;
-    double cdtd = dt;  // dt coefficient of the stage, FP64
-    bool x1_u1 = false;
-    if (a.stage == 1) {
-        if (a.rk == kRkTvd2) { cA = 0.5f; cB = 0.5f; cdtd = 0.5 * dt; }
-        else { cA = 0.75f; cB = 0.25f; cdtd = 0.25 * dt; }
-    } else if (a.stage == 2) {
-        // cA + cB must be exactly 1 in FP32, else the deviation form scales the
-        // stored deviations by (cA + cB) every step: cB = fl(2/3), cA = 1 - cB
-        // (an exact FP32 subtraction).
-        cB = float(2.0 / 3.0);
-        cA = 1.0f - cB;
-        cdtd = (2.0 / 3.0) * dt;
-        x1_u1 = a.rk == kRkTvd3Ref;
-    }
-    if (kFeat & kSchemeU1) x1_u1 = true;
-    if (kFeat & kSchemeNoU1) x1_u1 = false;
-    const float cdt = float(cdtd);
-    // Stochastic rounding of the state that ends each step (the last stage), or
-    // of every stage (CFS_ROUND_STOCHASTIC_ALL); otherwise round to nearest.
-    // Rounding an intermediate stage to nearest leaves a small mass bias: its
-    // increments are dt times differences of FP32 fluxes, a coarse lattice on
-    // the stored grid, so the rounding errors do not average out.
-    const bool last_of_step = a.rk == kRkTvd2 ? a.stage == 1 : a.stage == 2;
-    const bool sr = Pol::kMixed && ((kFeat & kSchemeSr) || stage_rounds_stochastically(a.rounding, last_of_step));
-    const unsigned int step_seed = (a.P ? a.P->seed[a.parity] : a.seed) * 4u + static_cast<unsigned int>(a.stage);
+    const UpdateCoefs uc = update_coefs<Pol, kFeat>(a);
     // physical boundary faces: the cell's own flux (transmissive) or a precomputed one (Dirichlet)
     const bool lo_x = kEdge && physical_side(a, 0), hi_x = kEdge && physical_side(a, 1);
     const bool lo_y = kEdge && physical_side(a, 2), hi_y = kEdge && physical_side(a, 3);
     const C* const bfl = static_cast<const C*>(a.bflux);
     const uint8_t* const flags = kEdge ? a.cflags : nullptr;
-    double* const rhs_out = kExtra ? a.rhs : nullptr;
     const T* const rv_in = kExtra ? static_cast<const T*>(a.rv) : nullptr;
-    if (a.P && a.first_stage && seg == 0 && by == 0 && lane == 0) {
-        a.P->wmax[1 - a.parity] = 0ull;
-        a.P->t += dt;
-        a.P->dt_last = dt;
-        a.P->seed[1 - a.parity] = a.P->seed[a.parity] + 1u;
-    }
+    if (a.P && a.first_stage && seg == 0 && by == 0 && lane == 0) begin_step(a, uc.dt);
     const bool active_warp = j0 < L.ny;  // uniform per warp
-    const bool do_cfl = a.P && a.last_stage && a.P->use_cfl;  // read once: stores to `out` may alias P for the compiler
 
     auto load_row = [&](int r, C out[kVars]) {
         if (col_ok) {
@@ -741,6 +947,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
     for (int r = i0 - 1; active_warp && r <= i1; ++r) {
         const unsigned int f_r = f_next;
         f_next = load_flags(r + 1);
+        if (r == i1) let_next_in();
         if constexpr (kRing && !kU0Ring) {  // FP64 ring: U^0 of row r-1, ahead of the x reconstruction
             if (a.stage >= 1 && owner && r - 1 >= i0) ld_cell<T>(static_cast<const T*>(a.u0), L.offset(r - 1, j), pf_u0);
         }
@@ -788,17 +995,10 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
             // branch of its own would not overlap the surrounding work)
             hll_flux<Pol>(Lx, Rr, 0, hll, g, FX);
             if ((r == 0 && lo_x) || (r == L.nx && hi_x)) {  // uniform per warp
-                // (no side index computed at run time: it would put the batch's argument block into local memory)
-                if (r == 0 ? a.bc[0] == kNeumann : a.bc[1] == kNeumann) {
-                    C c[kVars];
-                    if (r == 0) full(win[2], c);
-                    else full(win[1], c);
-                    wall_flux<Pol>(c, 0, g, FX);
-                } else if (j >= 0 && j < L.ny) {
-                    const C* b = bfl + bflux_side_offset(L, r == 0 ? 0 : 1);
-#pragma unroll
-                    for (int v = 0; v < kVars; ++v) FX[v] = b[static_cast<long long>(v) * L.ny + j];
-                }
+                C c[kVars];
+                if (r == 0) full(win[2], c);
+                else full(win[1], c);
+                boundary_x_flux<Pol>(a, r, j, c, FX);
             }
             // ---- update of row r-1 (its upper x-face is r - 1/2)
             const int i = r - 1;
@@ -815,94 +1015,14 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
                     load_update(i);
                 }
                 const bool fluid = !kEdge || !(f_prev & kCellSolid);
-                T* out = static_cast<T*>(a.out);
                 T u1c[kVars] = {T(0), T(0), T(0), T(0)};  // U^1 (TVD3 as written, stage 2 only)
-                if (x1_u1) ld_cell<T>(static_cast<const T*>(a.u1), L.offset(i, j), u1c);
-                C nv[kVars];  // new state in the form's arithmetic type, for the CFL maximum
-                T sv[kVars];
-                if constexpr (Pol::kMixed) {
-                    // FP32 update of the stored deviations (value - off): the RK
-                    // coefficients of a stage sum to 1, so the offsets cancel and
-                    // the rounding step is that of the deviation.
-                    // (formed for every cell and selected: a non-fluid cell keeps its state)
-                    float rvf[kVars], x0[kVars], x1[kVars], ndv[kVars];
+                if (uc.x1_u1) ld_cell<T>(static_cast<const T*>(a.u1), L.offset(i, j), u1c);
+                if constexpr (!Pol::kMixed && !kRing) {
 #pragma unroll
-                    for (int v = 0; v < kVars; ++v) {
-                        rvf[v] = -(FX[v] - FXp[v]) * inv_dxf + RY[v];
-                        if (kExtra && rv_in && v >= 1) rvf[v] += rv_cur[v - 1];
-                        x0[v] = (kU0Ring || a.stage >= 1) ? pf_u0[v] : pf_cur[v];
-                        // (stage 0: cB = 0 and x1 - x0 = 0, so x1 adds nothing)
-                        x1[v] = x1_u1 ? u1c[v] : pf_cur[v];
-                    }
-                    if (sr) {
-                        // Stochastic rounding of x0 + cB (x1 - x0) + cdt R (cA = 1 - cB
-                        // exactly): the increment is formed first, at its own
-                        // spacing (roundings near 1e-12 of the state, far below the
-                        // stored spacing), gets a dither uniform over one stored
-                        // spacing of the result's binade, and is added to x0 with
-                        // one rounding; two variables per packed instruction.
-                        const unsigned int h = cell_hash(i, j, step_seed);
-                        const float u[kVars] = {dither_bits<0>(h), dither_bits<1>(h), dither_bits<2>(h), dither_bits<3>(h)};
-#pragma unroll
-                        for (int v = 0; v < kVars; v += 2) {
-                            const float2 a0 = make_float2(x0[v], x0[v + 1]);
-                            const float2 inc = fma2(p2(cB), sub2(make_float2(x1[v], x1[v + 1]), a0),
-                                                    mul2(p2(cdt), make_float2(rvf[v], rvf[v + 1])));
-                            const float2 f = add2(a0, inc);
-                            const float2 t = add2(make_float2(u[v], u[v + 1]), p2(-kDitherCentre));
-                            const float2 r = add2(a0, fma2(make_float2(binade(f.x), binade(f.y)), t, inc));
-                            ndv[v] = r.x;
-                            ndv[v + 1] = r.y;
-                        }
-                    } else {
-#pragma unroll
-                        for (int v = 0; v < kVars; ++v) ndv[v] = fmaf(cdt, rvf[v], fmaf(cA, x0[v], cB * x1[v]));
-                    }
-#pragma unroll
-                    for (int v = 0; v < kVars; ++v) {
-                        const float cur = pf_cur[v];
-                        const float nd = fluid ? ndv[v] : cur;
-                        sv[v] = nd;
-                        nv[v] = nd + L.off[v];
-                        if (kExtra && rhs_out)
-                            rhs_out[static_cast<long long>(v) * L.nx * L.ny + static_cast<long long>(i) * L.ny + j] = fluid ? double(rvf[v]) : 0.0;
-                    }
-                } else {
-#pragma unroll
-                    for (int v = 0; v < kVars; ++v) {
-                        double rv = -double(FX[v] - FXp[v]) * inv_dx + double(RY[v]);
-                        if (kExtra && rv_in && v >= 1) rv += double(rv_cur[v - 1]);
-                        const double cur = double(win[1][v]);
-                        const double u0v = a.stage >= 1 ? dec<T>(pf_u0[v], L, v) : 0.0;
-                        const double u1v = x1_u1 ? dec<T>(u1c[v], L, v) : 0.0;
-                        const double val = fluid ? rk_update(a.rk, a.stage, dt, cur, u0v, u1v, rv) : cur;
-                        sv[v] = enc<T>(val, L, v);
-                        nv[v] = C(dec<T>(sv[v], L, v));
-                        if (kExtra && rhs_out)
-                            rhs_out[static_cast<long long>(v) * L.nx * L.ny + static_cast<long long>(i) * L.ny + j] = fluid ? rv : 0.0;
-                    }
+                    for (int v = 0; v < kVars; ++v) pf_cur[v] = T(win[1][v]);
                 }
-                if (kPos && a.positivity >= kPosFloor && fluid) {
-                    // p > floor, multiplied by rho > 0: (g-1)(rho E - |m|^2/2) > floor rho
-                    const C q = nv[3] * nv[0] - C(0.5) * (nv[1] * nv[1] + nv[2] * nv[2]);
-                    if (!(nv[0] > C(kRhoFloor)) || !(C(g - 1.0) * q > C(kPFloor) * nv[0])) {
-                        double s[kVars];
-#pragma unroll
-                        for (int v = 0; v < kVars; ++v)
-                            s[v] = Pol::kMixed ? double(sv[v]) + double(L.off[v]) : double(nv[v]);
-                        floor_state(s, g);
-#pragma unroll
-                        for (int v = 0; v < kVars; ++v) {
-                            sv[v] = Pol::kMixed ? T(s[v] - double(L.off[v])) : T(s[v]);
-                            nv[v] = C(s[v]);
-                        }
-                    }
-                }
-                store_cell4<T>(out, L, a.bc, i, j, sv);
-                if (do_cfl) {
-                    const double w = cfl_term(double(wave_sum_fast<C>(nv[0], nv[1], nv[2], nv[3], C(g), C(inv_dx), C(inv_dy))));
-                    if (fluid && w > wloc) wloc = w;
-                }
+                update_cell<Pol, kFeat>(a, uc, i, j, FX, FXp, RY, rv_cur, pf_cur,
+                                        (kU0Ring || a.stage >= 1) ? pf_u0 : pf_cur, u1c, fluid, wloc);
             }
         }
         // ---- y work of row r
@@ -923,43 +1043,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
 #pragma unroll
                 for (int k = 0; k < 5; ++k) get_slot<C>(rb[lane + k], st[k]);
             }
-            Face5<C> Ly, Ry;
-            cell_states<Pol>(st, eps, g, Ly, Ry, (kRing && Pol::kMixed) ? L.off : nullptr);
-            if constexpr (kPos) {
-                C cc[kVars];
-                full(st[2], cc);
-                fix_states<Pol>(f_r & kCellLowYhi, f_r & kCellLowYlo, cc, g, Ly, Ry);
-            }
-            // right state of the cell above (lane + 1)
-            Face5<C> Rn;
-            Rn.r = __shfl_down_sync(0xffffffffu, Ry.r, 1);
-            Rn.mx = __shfl_down_sync(0xffffffffu, Ry.mx, 1);
-            Rn.my = __shfl_down_sync(0xffffffffu, Ry.my, 1);
-            Rn.E = __shfl_down_sync(0xffffffffu, Ry.E, 1);
-            Rn.p = __shfl_down_sync(0xffffffffu, Ry.p, 1);
-            Rn.a = __shfl_down_sync(0xffffffffu, Ry.a, 1);
-            Rn.ri = __shfl_down_sync(0xffffffffu, Ry.ri, 1);
-            // face between column j and j+1 (face index j+1)
-            C FY[kVars];
-            hll_flux<Pol>(Ly, Rn, 1, hll, g, FY);
-            if (warp_ybnd && ybnd) {
-                if (bfy) {
-#pragma unroll
-                    for (int v = 0; v < kVars; ++v) FY[v] = bfy[static_cast<long long>(v) * L.nx + r];
-                } else {  // the interior cell: column 0 for the lane below it, this lane's at the top
-                    C c[kVars];
-#pragma unroll
-                    for (int v = 0; v < kVars; ++v) c[v] = j == -1 ? st[3][v] : st[2][v];
-                    full(c, c);
-                    wall_flux<Pol>(c, 1, g, FY);
-                }
-            }
-#pragma unroll
-            for (int v = 0; v < kVars; ++v) {
-                const C below = __shfl_up_sync(0xffffffffu, FY[v], 1);
-                if constexpr (Pol::kMixed) RY[v] = (below - FY[v]) * inv_dyf;  // as the x part: FP32
-                else RY[v] = C(-double(FY[v] - below) * inv_dy);
-            }
+            y_part<Pol, kFeat, kRing && Pol::kMixed>(a, uc, r, j, hll, st, eps, f_r, warp_ybnd, ybnd, bfy, RY);
             __syncwarp();
         }
         // ---- carry to the next row
@@ -1000,14 +1084,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
     } else if constexpr (kRing) {
         cp_async_wait_all();  // no copy into the ring outlives the item
     }
-    // CFL maximum: one atomic per warp (no block barrier, so the warps of a
-    // block never wait for each other)
-    if (do_cfl) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) wloc = fmax(wloc, __shfl_xor_sync(0xffffffffu, wloc, o));
-        if (lane == 0 && wloc > 0.0)
-            atomicMax(&a.P->wmax[1 - a.parity], static_cast<unsigned long long>(__double_as_longlong(wloc)));
-    }
+    if (uc.do_cfl) raise_wmax(a, wloc);
     return true;
 }
 
@@ -1041,6 +1118,7 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) march_kernel(const __
     const long long gw = static_cast<long long>(blockIdx.x) * kWarps + wid;
     const int seg = gw < nitems ? static_cast<int>(gw % nseg) : nseg;
     const int by = gw < nitems ? static_cast<int>(gw / nseg) : 0;
+    after_previous();
     // (the ring forms use no row buffer)
     __shared__ __align__(16) typename Pol::C rbuf[kLoad >= 3 ? 1 : kWarps][36][kVars];
     using RB = typename Pol::C(&)[kWarps][36][kVars];
@@ -1097,6 +1175,8 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks)
     typename Pol::T* const ring = kDynRing ? reinterpret_cast<typename Pol::T*>(batch_dyn_smem) : ring_static;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     unsigned int* const counter = counters + slot;
+    let_next_in();
+    after_previous();
     if (blockIdx.x == 0 && threadIdx.x < kBatchCounters && threadIdx.x / kBatchMaxGroups != slot / kBatchMaxGroups)
         counters[threadIdx.x] = 0u;  // the other stages' (see kBatchCounters)
     C(&wbuf)[1][36][kVars] = *reinterpret_cast<C(*)[1][36][kVars]>(&rbuf[kRing ? 0 : wid]);

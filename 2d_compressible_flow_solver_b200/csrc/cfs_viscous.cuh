@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(32 * kViscWarps, kMinBlocks) viscous_kernel(co
     const int nseg = (L.ny + kViscSeg - 1) / kViscSeg;
     const long long gw = static_cast<long long>(blockIdx.x) * kViscWarps + wid;
     const int i0 = static_cast<int>(gw / nseg) * a.rows;
+    let_next_in();
+    after_previous();
     if (i0 >= L.nx) return;  // (a warp past the last item; nothing below is block-wide)
     const int i1 = min(i0 + a.rows, L.nx);
     const int j = static_cast<int>(gw % nseg) * kViscSeg - 3 + lane;  // this lane's column

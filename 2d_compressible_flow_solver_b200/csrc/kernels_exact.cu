@@ -20,25 +20,21 @@ inline int flat_blocks(long long work, int nt) {
 }  // namespace
 
 cudaError_t launch_stage_exact(const StageArgs& a, cudaStream_t s) {
-    stage_kernel<PolExact, kTileI, kTileJ><<<stage_grid(a.L), kTileI * kTileJ, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_after(stage_kernel<PolExact, kTileI, kTileJ>, stage_grid(a.L), kTileI * kTileJ, 0, s, a);
 }
 
 cudaError_t launch_ib_fill(int elem_bytes, const IbArgs& a, cudaStream_t s) {
     if (a.n <= 0) return cudaSuccess;
     const int nt = 128, nb = (a.n + nt - 1) / nt;
-    if (elem_bytes == 8) ib_fill_kernel<double><<<nb, nt, 0, s>>>(a);
-    else ib_fill_kernel<float><<<nb, nt, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_after(elem_bytes == 8 ? ib_fill_kernel<double> : ib_fill_kernel<float>, nb, nt, 0, s, a);
 }
 
 cudaError_t launch_batch_ib_fill(int elem_bytes, const IbArgs* args, const int* cases, const int* local, int total,
                                  cudaStream_t s) {
     if (total <= 0) return cudaSuccess;
     const int nt = 128, nb = (total + nt - 1) / nt;
-    if (elem_bytes == 8) batch_ib_fill_kernel<double><<<nb, nt, 0, s>>>(args, cases, local, total);
-    else batch_ib_fill_kernel<float><<<nb, nt, 0, s>>>(args, cases, local, total);
-    return cudaGetLastError();
+    return launch_after(elem_bytes == 8 ? batch_ib_fill_kernel<double> : batch_ib_fill_kernel<float>, nb, nt, 0, s, args,
+                        cases, local, total);
 }
 
 cudaError_t launch_wmax(int elem_bytes, const void* U, const Layout& L, const uint8_t* types, double g, double dx,

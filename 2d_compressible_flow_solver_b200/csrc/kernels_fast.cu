@@ -1,11 +1,11 @@
 // Kernels of the throughput forms: FP64 with FMA contraction and the
 // FP32-mixed form.  Built with FMA contraction on (nvcc default).
 #include <atomic>
-#include <mutex>
 
 #include "cfs_kernels.cuh"
 #include "cfs_launch.h"
 #include "cfs_march.cuh"
+#include "cfs_resident.h"
 #include "cfs_viscous.cuh"
 
 namespace cfs {
@@ -17,11 +17,10 @@ cudaError_t launch_boundary_flux(const StageArgs& a, cudaStream_t s) {
     if (!dirichlet_side(a.bc)) return cudaSuccess;
     if (!a.bflux) return cudaErrorInvalidValue;
     const int n = a.L.nx > a.L.ny ? a.L.nx : a.L.ny;
-    boundary_flux_kernel<Pol><<<dim3((n + 127) / 128, 4), 128, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_after(boundary_flux_kernel<Pol>, dim3((n + 127) / 128, 4), 128, 0, s, a);
 }
 
-constexpr int kMaxDev = 64;
+constexpr int kMaxDev = ResidentCache::kMaxDev;
 
 // SM count of the current device (cached per device).
 int sm_count() {
@@ -110,9 +109,8 @@ cudaError_t launch_batch_kernel(const StageArgs* args, const int* item_case, con
     constexpr size_t dyn = batch_dyn_bytes<Pol, kLoad>();
     const cudaError_t e = allow_dyn(batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeat>, dyn);
     if (e != cudaSuccess) return e;
-    batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeat><<<grid, 32 * kBatchWarps, dyn, s>>>(
-        args, item_case, item_local, case_rows, case_nseg, total, counters, slot);
-    return cudaGetLastError();
+    return launch_after(batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeat>, grid, 32 * kBatchWarps, dyn, s, args,
+                        item_case, item_local, case_rows, case_nseg, total, counters, slot);
 }
 
 template <class Pol, int kMinBlocks, int kLoad, int kScheme, class... Args>
@@ -154,9 +152,8 @@ cudaError_t launch_batch_boundary_flux(Prec p, const StageArgs* args, int ncases
     for (int c0 = 0; c0 < ncases; c0 += 65535) {  // gridDim.z limit
         const int nc = ncases - c0 < 65535 ? ncases - c0 : 65535;
         const dim3 grid((max_edge + 127) / 128, 4, nc);
-        if (p == kF32Mixed) batch_boundary_flux_kernel<PolF32><<<grid, 128, 0, s>>>(args + c0);
-        else batch_boundary_flux_kernel<PolF64><<<grid, 128, 0, s>>>(args + c0);
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_after(p == kF32Mixed ? batch_boundary_flux_kernel<PolF32> : batch_boundary_flux_kernel<PolF64>,
+                                           grid, 128, 0, s, args + c0);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -182,32 +179,14 @@ int batch_blocks_per_sm(Prec p) {
 // x-face formed).
 template <class Pol, int kMinBlocks>
 cudaError_t launch_viscous_form(const ViscArgs& a_in, cudaStream_t s) {
-    static std::once_flag once[kMaxDev];
-    static long long slots_of[kMaxDev];
-    auto query = []() -> long long {
-        int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, viscous_kernel<Pol, kMinBlocks>, 32 * kViscWarps, 0) != cudaSuccess) {
-            (void)cudaGetLastError();  // a failed query leaves no error behind
-            return 0;
-        }
-        return static_cast<long long>(per_sm) * sm_count();
-    };
-    int dev = 0;
-    const cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    long long slots = 0;
-    if (dev < 0 || dev >= kMaxDev) {
-        slots = query();
-    } else {
-        std::call_once(once[dev], [&] { slots_of[dev] = query(); });
-        slots = slots_of[dev];
-    }
+    static ResidentCache cache;
+    const long long slots = resident_blocks(cache, viscous_kernel<Pol, kMinBlocks>, 32 * kViscWarps, 0);
     ViscArgs a = a_in;
     const int nseg = (a.L.ny + kViscSeg - 1) / kViscSeg;
     a.rows = slots > 0 ? choose_rows(nseg, kViscWarps, a.L.nx, slots) : 32;
     const long long items = static_cast<long long>(nseg) * ((a.L.nx + a.rows - 1) / a.rows);
-    viscous_kernel<Pol, kMinBlocks><<<static_cast<unsigned>((items + kViscWarps - 1) / kViscWarps), 32 * kViscWarps, 0, s>>>(a);
-    return cudaGetLastError();
+    const long long blocks = (items + kViscWarps - 1) / kViscWarps;
+    return launch_after(viscous_kernel<Pol, kMinBlocks>, static_cast<unsigned>(blocks), 32 * kViscWarps, 0, s, a);
 }
 
 cudaError_t launch_viscous_f64(const ViscArgs& a, cudaStream_t s) { return launch_viscous_form<PolF64, 3>(a, s); }
