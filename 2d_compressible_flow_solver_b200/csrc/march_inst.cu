@@ -8,6 +8,7 @@
 #include "cfs_launch.h"
 #include "cfs_march.cuh"
 #include "cfs_resident.h"
+#include "cfs_tile.cuh"
 
 #if !defined(CFS_MARCH_POL) || !defined(CFS_MARCH_FEAT) || !defined(CFS_MARCH_FN)
 #error "march_inst.cu needs CFS_MARCH_POL, CFS_MARCH_FEAT and CFS_MARCH_FN"
@@ -74,16 +75,49 @@ cudaError_t launch_march_k(const StageArgs& a, cudaStream_t s) {
     return launch_march<Pol, v.rows, v.warps, v.min_blocks, v.load, F>(a, s);
 }
 
+// The tile form with W warps per block, when its blocks fit `rounds` times on
+// the device; false: not launched.
+template <class Pol, int W, int F>
+bool launch_tile(const StageArgs& a, int rounds, cudaStream_t s, cudaError_t& e) {
+    auto kernel = tile_kernel<Pol, W, tile_min_blocks<typename Pol::T>(W), F>;
+    static ResidentCache cache;
+    const long long slots = resident_blocks(cache, kernel, 32 * W, 0);
+    const int nseg = (a.L.ny + kSeg - 1) / kSeg;
+    const int nrows = stage_row_hi(a) - stage_row_lo(a);
+    const long long blocks = static_cast<long long>(nseg) * ((nrows + W - 3) / (W - 2));
+    if (blocks > rounds * slots) return false;
+    e = nrows <= 0 ? cudaSuccess : launch_after(kernel, dim3(static_cast<unsigned>(blocks)), 32 * W, 0, s, a);
+    return true;
+}
+
+// A grid too small to fill the GPU runs in the tile form: the smaller tile
+// while all its blocks are resident at once, the larger one up to two rounds
+// of it; others march.  SSP3 steps (us) with the march / 4 warps / 10 (FP32)
+// or 8 (FP64) warps: FP32 periodic 64^2 14.3 / 11.3 / 12.5, 160^2 17.4 / 15.1 /
+// 15.0, 256^2 21.4 / 22.7 / 16.3, 352^2 29.7 / 33.7 / 26.9, 384^2 30.7 / 39.8 /
+// 33.4; FP64 64^2 18.4 / 13.4 / 15.4, 192^2 29.7 / 27.0 / 22.4, 352^2 46.0 /
+// 53.8 / 43.8, 384^2 46.1 / 60.1 / 50.4; cylinder 400 x 200 FP32 43.2 / 46.0 /
+// 39.3, FP64 59.3 / 60.1 / 54.5.  A caller that fixes the march's rows or
+// variant gets the march (the same bits).
+template <class Pol, int K, int F>
+cudaError_t launch_default_scheme(const StageArgs& a, cudaStream_t s) {
+    if (a.rows == 0 && a.variant == 0) {
+        cudaError_t e = cudaSuccess;
+        if (launch_tile<Pol, 4, F>(a, 1, s, e) || launch_tile<Pol, Pol::kMixed ? 10 : 8, F>(a, 2, s, e)) return e;
+    }
+    return launch_march_k<Pol, K, F>(a, s);
+}
+
 // The variant that runs by default, with the launch's scheme compiled in.
 template <class Pol, int K, int F>
 cudaError_t launch_march_default(const StageArgs& a, cudaStream_t s) {
     const bool last_of_step = a.stage == (a.rk == kRkTvd2 ? 1 : 2);
     const bool sr = !Pol::kMixed || stage_rounds_stochastically(a.rounding, last_of_step);
     switch (known_scheme(a.hll == kHllDavis, a.rk == kRkTvd3Ref, a.stage, sr)) {
-        case kScheme0: return launch_march_k<Pol, K, F | kScheme0>(a, s);
-        case kScheme1: return launch_march_k<Pol, K, F | kScheme1>(a, s);
-        case kScheme2: return launch_march_k<Pol, K, F | kScheme2>(a, s);
-        default: return launch_march_k<Pol, K, F>(a, s);
+        case kScheme0: return launch_default_scheme<Pol, K, F | kScheme0>(a, s);
+        case kScheme1: return launch_default_scheme<Pol, K, F | kScheme1>(a, s);
+        case kScheme2: return launch_default_scheme<Pol, K, F | kScheme2>(a, s);
+        default: return launch_default_scheme<Pol, K, F>(a, s);
     }
 }
 
