@@ -54,6 +54,7 @@ struct cfs_ctx {
     std::vector<uint8_t> types_h;
     // immersed ghosts
     int ib_n = 0, ib_mode = 0;
+    bool ib_at_edge = false;  // an immersed-ghost cell lies next to a side of the grid
     int* ib_cell = nullptr;
     int* ib_donor = nullptr;
     int* ib_perm = nullptr;
@@ -256,7 +257,14 @@ Roles roles_for(const cfs_ctx* c, int stage, int cur, int u0_idx, int u1_idx) {
 // select graph mode.
 int enqueue_stage(cfs_ctx* c, int stage, const Roles& r, double dt, bool graph_mode, int parity, bool first,
                   bool last, int row_lo = 0, int row_hi = 0, bool with_fill = true) {
-    if (with_fill && c->ib_n > 0) CFS_CUDA(c, cfs::launch_ib_fill(c->L.elem_bytes, ib_args(c, c->S[r.in]), c->stream));
+    cfs::StageArgs a = base_args(c);
+    a.in = c->S[r.in];
+    const bool fill = with_fill && c->ib_n > 0, faces = c->prec != cfs::kF64Exact && cfs::dirichlet_side(c->cfg.bc);
+    if (fill && (!faces || c->ib_at_edge)) CFS_CUDA(c, cfs::launch_ib_fill(c->L.elem_bytes, ib_args(c, c->S[r.in]), c->stream));
+    if (faces) {
+        const cfs::IbArgs ib = ib_args(c, c->S[r.in]);
+        CFS_CUDA(c, cfs::launch_pre_stage(c->prec, fill && !c->ib_at_edge ? &ib : nullptr, &a, c->stream));
+    }
     if (c->rv && with_fill) {
         cfs::ViscArgs va{};
         va.in = c->S[r.in];
@@ -278,9 +286,7 @@ int enqueue_stage(cfs_ctx* c, int stage, const Roles& r, double dt, bool graph_m
         va.inv_dy_f = static_cast<float>(va.inv_dy);
         CFS_CUDA(c, cfs::launch_viscous(c->prec, va, c->stream));
     }
-    cfs::StageArgs a = base_args(c);
     a.rv = c->rv;
-    a.in = c->S[r.in];
     a.u0 = r.u0 >= 0 ? c->S[r.u0] : nullptr;
     a.u1 = r.u1 >= 0 ? c->S[r.u1] : nullptr;
     a.out = c->S[r.out];
@@ -362,6 +368,7 @@ int upload_ib(cfs_ctx* c, int mode, int n, const int32_t* cell, const int32_t* d
     CFS_CUDA(c, cudaMemcpy(c->ib_fac, fac.data(), sizeof(double) * 16 * n, cudaMemcpyHostToDevice));
     c->ib_n = n;
     c->ib_mode = mode;
+    c->ib_at_edge = cfs::ib_at_edge(n, cell, c->cfg.nx, c->cfg.ny);
     return CFS_OK;
 }
 

@@ -64,6 +64,7 @@ struct cfs_batch {
     std::vector<FeatureGroup> groups;  // work items by feature set, largest cases first in each
     int max_edge = 0;        // largest nx or ny of the cases
     int total_ig = 0;
+    bool ib_at_edge = false;  // some immersed-ghost cell lies next to a side of its grid
     int* ib_cell = nullptr;
     int* ib_donor = nullptr;
     int* ib_perm = nullptr;
@@ -225,12 +226,18 @@ int enqueue_batch_step(cfs_batch* b, int parity) {
         const int scheme = cfs::known_scheme(
             b->common.hll == CFS_HLL_DAVIS, b->common.rk == CFS_RK_TVD3_REFERENCE, s,
             b->prec != cfs::kF32Mixed || cfs::stage_rounds_stochastically(b->common.rounding, s == S - 1));
-        if (b->total_ig > 0)
-            CFSB_CUDA(b, cfs::launch_batch_ib_fill(b->elem, b->dib + static_cast<size_t>(in) * b->n, b->ig_case,
-                                                   b->ig_local, b->total_ig, b->stream));
-        if (b->any_bflux)
-            CFSB_CUDA(b, cfs::launch_batch_boundary_flux(b->prec, b->dargs + static_cast<size_t>(slot) * b->n, b->n,
-                                                         b->max_edge, b->stream));
+        const cfs::StageArgs* const args = b->dargs + static_cast<size_t>(slot) * b->n;
+        auto pre = [&](int total, int ncases) {
+            return cfs::launch_batch_pre_stage(b->prec, b->dib + static_cast<size_t>(in) * b->n, b->ig_case, b->ig_local, total,
+                                               args, ncases, b->max_edge, b->stream);
+        };
+        const int face_cases = b->any_bflux ? b->n : 0;
+        if (b->ib_at_edge && face_cases > 0) {  // a face flux may read a ghost: fill first
+            CFSB_CUDA(b, pre(b->total_ig, 0));
+            CFSB_CUDA(b, pre(0, face_cases));
+        } else {
+            CFSB_CUDA(b, pre(b->total_ig, face_cases));
+        }
         for (size_t g = 0; g < b->groups.size(); ++g) {
             const FeatureGroup& fg = b->groups[g];
             CFSB_CUDA(b, cfs::launch_batch_stage(b->prec, b->dargs + static_cast<size_t>(slot) * b->n,
@@ -380,6 +387,7 @@ int cfs_batch_create(const cfs_config* common, int ncases, const cfs_case* cases
             std::vector<int> perm;
             cfs::ib_factors(d.ib_mode, c.types.data(), d.nx, d.ny, c.dx, c.dy, c.ib_n, ib.donor.data(), ib.image.data(),
                             ib.normal.data(), dd, fac, perm);
+            b->ib_at_edge = b->ib_at_edge || cfs::ib_at_edge(c.ib_n, ib.cell.data(), d.nx, d.ny);
             h_cell.insert(h_cell.end(), ib.cell.begin(), ib.cell.end());
             h_donor.insert(h_donor.end(), dd.begin(), dd.end());
             h_perm.insert(h_perm.end(), perm.begin(), perm.end());

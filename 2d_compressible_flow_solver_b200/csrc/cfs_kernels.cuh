@@ -283,7 +283,7 @@ __device__ __forceinline__ C weno5_fast(C v0, C v1, C v2, C v3, C v4, C eps) {
     const C p0 = C(2) * v0 - C(7) * v1 + C(11) * v2;
     const C p1 = -v1 + C(5) * v2 + C(2) * v3;
     const C p2 = C(2) * v2 + C(5) * v3 - v4;
-    return (a0 * p0 + a1 * p1 + a2 * p2) * rcp_fast(C(6) * (a0 + a1 + a2));
+    return (a0 * p0 + a1 * p1 + a2 * p2) * rcp_pos(C(6) * (a0 + a1 + a2));
 }
 
 template <class Pol>
@@ -844,19 +844,6 @@ __global__ void ib_fill_kernel(const IbArgs a) {
     after_previous();
     if (g >= a.n) return;
     ib_fill_one<T>(a, g);
-}
-
-// Batched form: immersed-ghost cell g of the batch is cell local[g] of case
-// cases[g]; args[c] is case c's fill description (its state buffer, layout, lists).
-template <class T>
-__global__ void batch_ib_fill_kernel(const IbArgs* __restrict__ args, const int* __restrict__ cases,
-                                     const int* __restrict__ local, int total) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    let_next_in();
-    after_previous();
-    if (g >= total) return;
-    const IbArgs a = args[cases[g]];
-    ib_fill_one<T>(a, local[g]);
 }
 
 // ------------------------------------------------------ CFL reduction

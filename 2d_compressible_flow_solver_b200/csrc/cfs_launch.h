@@ -17,6 +17,9 @@ constexpr int kTileJ = 32;
 
 cudaError_t launch_stage(Prec p, const StageArgs& a, cudaStream_t s);
 cudaError_t launch_ib_fill(int elem_bytes, const IbArgs& a, cudaStream_t s);
+// Before a stage of the throughput forms: the immersed-ghost fill (ib; null:
+// none) and the fluxes through the Dirichlet boundary faces (a; null: none).
+cudaError_t launch_pre_stage(Prec p, const IbArgs* ib, const StageArgs* a, cudaStream_t s);
 cudaError_t launch_wmax(int elem_bytes, const void* U, const Layout& L, const uint8_t* types, double g, double dx,
                         double dy, unsigned long long* out, cudaStream_t s);
 // CFL maxima of every case of a batch: args[c].in into args[c].P->wmax[0].
@@ -134,10 +137,10 @@ cudaError_t launch_batch_stage(Prec p, const StageArgs* args, const int* item_ca
                                const int* case_rows, const int* case_nseg, int total, unsigned int* counters,
                                int slot, int grid, int feat, int scheme,
                                cudaStream_t s);  // feat: kFeatPos | kFeatEdge bits; scheme: known_scheme
-// Boundary-face fluxes of every case (grid: max_edge = the largest nx or ny).
-cudaError_t launch_batch_boundary_flux(Prec p, const StageArgs* args, int ncases, int max_edge, cudaStream_t s);
-cudaError_t launch_batch_ib_fill(int elem_bytes, const IbArgs* args, const int* cases, const int* local, int total,
-                                 cudaStream_t s);
+// The same for a batch: the immersed-ghost cells of every case (total; may be
+// 0) and the Dirichlet faces of every case (ncases; 0: none).
+cudaError_t launch_batch_pre_stage(Prec p, const IbArgs* ibs, const int* cases, const int* local, int total,
+                                   const StageArgs* args, int ncases, int max_edge, cudaStream_t s);
 int batch_blocks_per_sm(Prec p);
 
 // Per-policy entry points behind the dispatchers above.

@@ -403,7 +403,7 @@ __device__ __forceinline__ void wall_flux(const typename Pol::C c[kVars], int di
 
 // Fluxes through the Dirichlet boundary faces of one stage (the reference's
 // boundary stencil [g g g | c c c], CellInterface.cpp:172-178, then the
-// positivity fallback and HLL), computed by boundary_flux_kernel before the
+// positivity fallback and HLL), computed by pre_stage_kernel before the
 // row march, which reads them (StageArgs::bflux) instead of reconstructing
 // there.  (Transmissive faces need no stencil: the march forms them itself,
 // wall_flux, which saves their grids this launch -- 3.8 us a stage at
@@ -455,27 +455,10 @@ __device__ __forceinline__ void boundary_face_flux(const StageArgs& a, int s, in
     for (int v = 0; v < kVars; ++v) out[static_cast<long long>(v) * n + k] = F[v];
 }
 
-// One thread per boundary face: blockIdx.y = side, threads over the face index.
+// Face k of side s when that is a Dirichlet side's.
 template <class Pol>
-__global__ void __launch_bounds__(128) boundary_flux_kernel(const StageArgs a) {
-    const int s = blockIdx.y;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    let_next_in();
-    after_previous();
-    if (a.bc[s] != kDirichlet || k >= (s < 2 ? a.L.ny : a.L.nx)) return;
-    boundary_face_flux<Pol>(a, s, k);
-}
-
-// Batched form: blockIdx.z = case (args[c]), blockIdx.y = side.
-template <class Pol>
-__global__ void __launch_bounds__(128) batch_boundary_flux_kernel(const StageArgs* __restrict__ args) {
-    const StageArgs& a = args[blockIdx.z];
-    const int s = blockIdx.y;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    let_next_in();
-    after_previous();
-    if (!a.bflux || a.bc[s] != kDirichlet || k >= (s < 2 ? a.L.ny : a.L.nx)) return;
-    boundary_face_flux<Pol>(a, s, k);
+__device__ __forceinline__ void maybe_boundary_flux(const StageArgs& a, int s, int k) {
+    if (a.bc[s] == kDirichlet && k < (s < 2 ? a.L.ny : a.L.nx)) boundary_face_flux<Pol>(a, s, k);
 }
 
 // What the update of a stage's cells shares.
@@ -739,7 +722,7 @@ __device__ __forceinline__ void y_part(const StageArgs& a, const UpdateCoefs& k,
 //
 // The row loop holds no rarely taken code of any size: a transmissive face's
 // flux is the cell's own (wall_flux), a Dirichlet one is read from
-// boundary_flux_kernel, and cell types and low-order faces
+// pre_stage_kernel, and cell types and low-order faces
 // come from one flag byte per cell (StageArgs::cflags), both compiled in only
 // with kFeatEdge; the positivity fallback is a select of the cell's own state
 // (kFeatPos); the RHS copy and viscous RHS come with kFeatExtra.  A loop body that outgrows the

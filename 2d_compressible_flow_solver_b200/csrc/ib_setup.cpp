@@ -388,4 +388,12 @@ std::vector<uint8_t> cell_flags(const uint8_t* types, const uint8_t* lowo, int n
     return f;
 }
 
+bool ib_at_edge(int n, const int32_t* cell, int nx, int ny) {
+    for (int g = 0; g < n; ++g) {
+        const int i = cell[g] / ny, j = cell[g] % ny;
+        if (i == 0 || i == nx - 1 || j == 0 || j == ny - 1) return true;
+    }
+    return false;
+}
+
 }  // namespace cfs

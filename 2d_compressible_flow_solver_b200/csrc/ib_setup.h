@@ -89,4 +89,7 @@ std::vector<uint8_t> low_order_faces(const uint8_t* types, int nx, int ny, const
 // its four faces.
 std::vector<uint8_t> cell_flags(const uint8_t* types, const uint8_t* lowo, int nx, int ny);
 
+// Whether one of n immersed-ghost cells (i*ny + j) lies next to a side of the grid.
+bool ib_at_edge(int n, const int32_t* cell, int nx, int ny);
+
 }  // namespace cfs

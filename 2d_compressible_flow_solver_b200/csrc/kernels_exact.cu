@@ -4,6 +4,7 @@
 // ghost fill, the CFL reduction and the layout helpers for both storage types.
 #include "cfs_kernels.cuh"
 #include "cfs_launch.h"
+#include "cfs_march.cuh"
 #include "cfs_resident.h"
 
 namespace cfs {
@@ -37,12 +38,71 @@ cudaError_t launch_ib_fill(int elem_bytes, const IbArgs& a, cudaStream_t s) {
     return launch_after(elem_bytes == 8 ? ib_fill_kernel<double> : ib_fill_kernel<float>, nb, nt, 0, s, a);
 }
 
-cudaError_t launch_batch_ib_fill(int elem_bytes, const IbArgs* args, const int* cases, const int* local, int total,
-                                 cudaStream_t s) {
-    if (total <= 0) return cudaSuccess;
-    const int nt = 128, nb = (total + nt - 1) / nt;
-    return launch_after(elem_bytes == 8 ? batch_ib_fill_kernel<double> : batch_ib_fill_kernel<float>, nb, nt, 0, s, args,
-                        cases, local, total);
+// What a stage of the throughput forms needs before its march, in one launch:
+// the immersed-ghost fill (blocks below ib_blocks; n cells) and the fluxes
+// through the Dirichlet boundary faces (face_blocks blocks of 128 faces per
+// side).  Both are chains of a few microseconds on a few blocks; in two launches
+// they cost the 605 x 301 FP64 cylinder 10 of a stage's 27 us (step 79.9 -> 73.1
+// us; 2048 x 1024 FP32 258 -> 251, the uneven batch 901 -> 889).  A face flux reads the
+// cells next to its side, so a body whose ghosts lie there fills first, in a
+// launch of its own.
+constexpr int kPreThreads = 128;
+template <class Pol>
+__global__ void __launch_bounds__(kPreThreads) pre_stage_kernel(const IbArgs ib, const __grid_constant__ StageArgs a,
+                                                                int ib_blocks, int face_blocks) {
+    const int b = static_cast<int>(blockIdx.x), t = static_cast<int>(threadIdx.x);
+    let_next_in();
+    after_previous();
+    if (b < ib_blocks) {
+        if (b * kPreThreads + t < ib.n) ib_fill_one<typename Pol::T>(ib, b * kPreThreads + t);
+    } else {
+        maybe_boundary_flux<Pol>(a, (b - ib_blocks) / face_blocks, (b - ib_blocks) % face_blocks * kPreThreads + t);
+    }
+}
+
+cudaError_t launch_pre_stage(Prec p, const IbArgs* ib, const StageArgs* a, cudaStream_t s) {
+    static const StageArgs no_faces{};
+    const int ib_blocks = ib ? (ib->n + kPreThreads - 1) / kPreThreads : 0;
+    const int n = !a ? 0 : a->L.nx > a->L.ny ? a->L.nx : a->L.ny;
+    const int face_blocks = (n + kPreThreads - 1) / kPreThreads;
+    const int blocks = ib_blocks + 4 * face_blocks;
+    if (blocks == 0) return cudaSuccess;
+    if (a && !a->bflux) return cudaErrorInvalidValue;
+    return launch_after(p == kF32Mixed ? pre_stage_kernel<PolF32> : pre_stage_kernel<PolF64>, blocks, kPreThreads, 0, s,
+                        ib ? *ib : IbArgs{}, a ? *a : no_faces, ib_blocks, face_blocks);
+}
+
+// Batched form: immersed-ghost cell g of the batch is cell local[g] of case
+// cases[g] (ibs[c]: case c's fill description); the faces of every case with a
+// Dirichlet side (args[c].bflux; face_blocks covers the largest edge).
+template <class Pol>
+__global__ void __launch_bounds__(kPreThreads) batch_pre_stage_kernel(const IbArgs* __restrict__ ibs, const int* __restrict__ cases,
+                                                                      const int* __restrict__ local, int total, int ib_blocks,
+                                                                      const StageArgs* __restrict__ args, int face_blocks) {
+    const int b = static_cast<int>(blockIdx.x), t = static_cast<int>(threadIdx.x);
+    let_next_in();
+    after_previous();
+    if (b < ib_blocks) {
+        const int g = b * kPreThreads + t;
+        if (g >= total) return;
+        const IbArgs ib = ibs[cases[g]];
+        ib_fill_one<typename Pol::T>(ib, local[g]);
+    } else {
+        const int f = b - ib_blocks, side = f / face_blocks;
+        const StageArgs& a = args[side / 4];
+        if (a.bflux) maybe_boundary_flux<Pol>(a, side % 4, f % face_blocks * kPreThreads + t);
+    }
+}
+
+cudaError_t launch_batch_pre_stage(Prec p, const IbArgs* ibs, const int* cases, const int* local, int total,
+                                   const StageArgs* args, int ncases, int max_edge, cudaStream_t s) {
+    const int ib_blocks = (total + kPreThreads - 1) / kPreThreads;
+    const int face_blocks = ncases > 0 ? (max_edge + kPreThreads - 1) / kPreThreads : 0;
+    const long long blocks = ib_blocks + 4LL * face_blocks * ncases;
+    if (blocks == 0) return cudaSuccess;
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+    return launch_after(p == kF32Mixed ? batch_pre_stage_kernel<PolF32> : batch_pre_stage_kernel<PolF64>,
+                        static_cast<unsigned>(blocks), kPreThreads, 0, s, ibs, cases, local, total, ib_blocks, args, face_blocks);
 }
 
 cudaError_t launch_wmax(int elem_bytes, const void* U, const Layout& L, const uint8_t* types, double g, double dx,

@@ -10,16 +10,6 @@
 
 namespace cfs {
 
-// Boundary-face fluxes of the stage (Dirichlet sides only), then the row march
-// of the stage's feature set.
-template <class Pol>
-cudaError_t launch_boundary_flux(const StageArgs& a, cudaStream_t s) {
-    if (!dirichlet_side(a.bc)) return cudaSuccess;
-    if (!a.bflux) return cudaErrorInvalidValue;
-    const int n = a.L.nx > a.L.ny ? a.L.nx : a.L.ny;
-    return launch_after(boundary_flux_kernel<Pol>, dim3((n + 127) / 128, 4), 128, 0, s, a);
-}
-
 constexpr int kMaxDev = ResidentCache::kMaxDev;
 
 // SM count of the current device (cached per device).
@@ -54,8 +44,6 @@ int default_variant_f64(const Layout& L, int rows) {
 }
 
 cudaError_t launch_stage_f64(const StageArgs& a, cudaStream_t s) {
-    const cudaError_t e = launch_boundary_flux<PolF64>(a, s);
-    if (e != cudaSuccess) return e;
     // (with the row chunk chosen per launch to fill whole waves, the ring
     // variant stays; the fallback serves fixed chunks)
     const int v = a.variant > 0 ? a.variant : a.rows > 0 ? default_variant_f64(a.L, a.rows) : kDefaultVariantF64;
@@ -72,8 +60,6 @@ cudaError_t launch_stage_f64(const StageArgs& a, cudaStream_t s) {
 }
 
 cudaError_t launch_stage_f32(const StageArgs& a, cudaStream_t s) {
-    const cudaError_t e = launch_boundary_flux<PolF32>(a, s);
-    if (e != cudaSuccess) return e;
     const int v = a.variant > 0 ? a.variant : kDefaultVariantF32;
     switch (march_features(a)) {
         case 0: return launch_march_f32_0(a, v, s);
@@ -144,19 +130,6 @@ cudaError_t launch_batch_stage(Prec p, const StageArgs* args, const int* item_ca
             scheme, feat, args, item_case, item_local, case_rows, case_nseg, total, counters, slot, grid, s);
     return launch_batch_scheme<PolF64, kBatchMinBlocksF64, kBatchLoadF64>(
         scheme, feat, args, item_case, item_local, case_rows, case_nseg, total, counters, slot, grid, s);
-}
-
-// Boundary-face fluxes of every case of a batch (cases without Dirichlet sides
-// carry no bflux and return at once).
-cudaError_t launch_batch_boundary_flux(Prec p, const StageArgs* args, int ncases, int max_edge, cudaStream_t s) {
-    for (int c0 = 0; c0 < ncases; c0 += 65535) {  // gridDim.z limit
-        const int nc = ncases - c0 < 65535 ? ncases - c0 : 65535;
-        const dim3 grid((max_edge + 127) / 128, 4, nc);
-        const cudaError_t e = launch_after(p == kF32Mixed ? batch_boundary_flux_kernel<PolF32> : batch_boundary_flux_kernel<PolF64>,
-                                           grid, 128, 0, s, args + c0);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
 }
 
 int batch_blocks_per_sm(Prec p) {
