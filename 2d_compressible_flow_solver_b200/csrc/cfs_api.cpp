@@ -68,7 +68,8 @@ struct cfs_ctx {
     double* totals = nullptr;
     cudaGraphExec_t graph2 = nullptr;  // two full steps (parity 0 then 1)
     cudaGraphExec_t graph1 = nullptr;  // one full step (parity 0): an odd step count's last step
-    cfs::DevParams* hp_pin = nullptr;  // pinned host copies of cfs_advance's parameters in [0] and results in [1]
+    cfs::HostResults* results = nullptr;  // pinned; behind it, for a small grid, its host-order state (small_state)
+    double* small_state = nullptr;        // null: states move by copies
     // device-ordered stepping (cfs_steps_*): between begin and end
     bool in_steps = false;
     bool steps_cfl = false;
@@ -78,6 +79,9 @@ struct cfs_ctx {
 };
 
 namespace {
+
+// States up to this size move through a pinned array made with the context.
+constexpr size_t kSmallStateBytes = 512 << 10;
 
 thread_local std::string g_create_error;
 
@@ -207,16 +211,22 @@ cfs::StageArgs base_args(const cfs_ctx* c) {
 
 // Device error flags set by bounded waits in the kernels; read (and cleared)
 // at the calls that wait for the stream.
-int check_device_errors(cfs_ctx* c) {
-    unsigned int e = 0;
-    CFS_CUDA(c, cudaMemcpyAsync(&e, c->err_d, sizeof(e), cudaMemcpyDeviceToHost, c->stream));
-    CFS_CUDA(c, cudaStreamSynchronize(c->stream));
+int report_device_errors(cfs_ctx* c, unsigned int e) {
     if (e != 0) {
         CFS_CUDA(c, cudaMemsetAsync(c->err_d, 0, sizeof(unsigned int), c->stream));
         return fail(c, CFS_ERR_CUDA, "a TMA row copy did not complete within its bounded wait (device flag " +
                                          std::to_string(e) + ")");
     }
     return CFS_OK;
+}
+
+// Waits for the stream and reads back its results: the step parameters (when
+// asked for) and the error flags.
+int wait_results(cfs_ctx* c, cfs::DevParams* params) {
+    CFS_CUDA(c, cfs::launch_results(c->results, params ? c->P : nullptr, nullptr, c->err_d, c->stream));
+    CFS_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (params) *params = c->results->params;
+    return report_device_errors(c, c->results->err);
 }
 
 cfs::IbArgs ib_args(const cfs_ctx* c, void* U) {
@@ -507,11 +517,15 @@ int cfs_create(const cfs_config* cfg, cfs_ctx** out) {
     }
     cudaMemsetAsync(c->P, 0, sizeof(cfs::DevParams), c->stream);
     cudaMemsetAsync(c->err_d, 0, sizeof(unsigned int), c->stream);
-    // (without it, cfs_advance copies its parameters through pageable memory)
-    if (cudaHostAlloc(&c->hp_pin, 2 * sizeof(cfs::DevParams), cudaHostAllocDefault) != cudaSuccess) {
-        (void)cudaGetLastError();
-        c->hp_pin = nullptr;
+    cudaMemsetAsync(c->wmax, 0, sizeof(unsigned long long), c->stream);
+    const size_t small = hb <= kSmallStateBytes ? hb : 0;
+    void* pinned = nullptr;
+    if (cudaHostAlloc(&pinned, sizeof(cfs::HostResults) + small, cudaHostAllocDefault) != cudaSuccess) {
+        c->err = "pinned host allocation of the results failed";
+        return bail(CFS_ERR_NOMEM);
     }
+    c->results = static_cast<cfs::HostResults*>(pinned);
+    if (small) c->small_state = reinterpret_cast<double*>(c->results + 1);
     if (c->prec != cfs::kF64Exact) {
         // tensor maps of the three state buffers (TMA load schedule), encoded
         // on the host once (the buffers never move) and passed in each
@@ -524,7 +538,7 @@ int cfs_create(const cfs_config* cfg, cfs_ctx** out) {
         }
         c->has_tmaps = true;
     }
-    for (int b = 0; b < 3; ++b) cfs::launch_ghost_fill(c->L.elem_bytes, c->S[b], c->L, c->sides, c->stream);
+    cfs::launch_ghost_fill(c->L.elem_bytes, c->S, c->L, c->sides, c->stream);
     // the clears and ghost fills above are checked here, at enqueue and at completion
     cudaError_t ie = cudaStreamSynchronize(c->stream);
     if (ie == cudaSuccess) ie = cudaGetLastError();
@@ -554,7 +568,7 @@ int cfs_destroy(cfs_ctx* c) {
     cudaFree(c->ib_img);
     cudaFree(c->ib_fac);
     cudaFree(c->P);
-    if (c->hp_pin) cudaFreeHost(c->hp_pin);
+    if (c->results) cudaFreeHost(c->results);
     cudaFree(c->wmax);
     cudaFree(c->totals);
     cudaFree(c->err_d);
@@ -601,17 +615,21 @@ int cfs_set_state(cfs_ctx* c, const double* U) {
     c->wmax_carry = false;
     CFS_CUDA(c, cudaSetDevice(c->cfg.device));
     const size_t hb = sizeof(double) * kVars * static_cast<size_t>(c->cfg.nx) * c->cfg.ny;
-    CFS_CUDA(c, copy_in(c, c->staging, U, hb));
+    if (c->small_state) {
+        std::memcpy(c->small_state, U, hb);
+        CFS_CUDA(c, cudaMemcpyAsync(c->staging, c->small_state, hb, cudaMemcpyHostToDevice, c->stream));
+    } else {
+        CFS_CUDA(c, copy_in(c, c->staging, U, hb));
+    }
     if (c->L.elem_bytes == 4) {
         // FP32 storage offsets: the FP32-rounded mean of each variable, summed
         // on the device from the uploaded state (a fixed summation order)
         const size_t n = static_cast<size_t>(c->cfg.nx) * c->cfg.ny;
         double sums[kVars] = {0, 0, 0, 0};
         if (!c->fixed_offsets) {
-            CFS_CUDA(c, cfs::launch_plane_sums(c->staging, static_cast<long long>(n), c->sums, c->stream));
-            CFS_CUDA(c, cudaMemcpyAsync(sums, c->sums + cfs::plane_sums_scratch_doubles() - kVars, sizeof(sums),
-                                        cudaMemcpyDeviceToHost, c->stream));
+            CFS_CUDA(c, cfs::launch_plane_sums(c->staging, static_cast<long long>(n), c->sums, c->results->sums, c->stream));
             CFS_CUDA(c, cudaStreamSynchronize(c->stream));
+            std::memcpy(sums, c->results->sums, sizeof(sums));
         }
         bool changed = false;
         for (int v = 0; v < kVars; ++v) {
@@ -623,7 +641,7 @@ int cfs_set_state(cfs_ctx* c, const double* U) {
         if (changed) release_graph(c);
     }
     CFS_CUDA(c, cfs::launch_pack(c->L.elem_bytes, c->staging, c->S[0], c->L, c->stream));
-    for (int b = 0; b < 3; ++b) CFS_CUDA(c, cfs::launch_ghost_fill(c->L.elem_bytes, c->S[b], c->L, c->sides, c->stream));
+    CFS_CUDA(c, cfs::launch_ghost_fill(c->L.elem_bytes, c->S, c->L, c->sides, c->stream));
     CFS_CUDA(c, cudaStreamSynchronize(c->stream));
     c->cur = 0;
     c->u0_idx = c->u1_idx = -1;
@@ -666,9 +684,17 @@ int cfs_get_state(cfs_ctx* c, double* U) {
     if (!c || !U) return fail(c, CFS_ERR_INVALID, "null argument");
     CFS_CUDA(c, cudaSetDevice(c->cfg.device));
     const size_t hb = sizeof(double) * kVars * static_cast<size_t>(c->cfg.nx) * c->cfg.ny;
-    CFS_CUDA(c, cfs::launch_unpack(c->L.elem_bytes, c->S[c->cur], c->staging, c->L, c->stream));
-    CFS_CUDA(c, copy_out(c, U, c->staging, hb));
-    return check_device_errors(c);
+    // a small state is written to the pinned array by the kernel itself
+    double* const dst = c->small_state ? c->small_state : c->staging;
+    CFS_CUDA(c, cfs::launch_unpack(c->L.elem_bytes, c->S[c->cur], dst, c->L, c->stream));
+    CFS_CUDA(c, cfs::launch_results(c->results, nullptr, nullptr, c->err_d, c->stream));
+    if (c->small_state) {
+        CFS_CUDA(c, cudaStreamSynchronize(c->stream));
+        std::memcpy(U, c->small_state, hb);
+    } else {
+        CFS_CUDA(c, copy_out(c, U, c->staging, hb));
+    }
+    return report_device_errors(c, c->results->err);
 }
 
 int cfs_get_rhs(cfs_ctx* c, double* R) {
@@ -853,14 +879,12 @@ int cfs_compute_dt(cfs_ctx* c, double cfl, double* dt) {
     if (!c || !dt) return fail(c, CFS_ERR_INVALID, "null argument");
     if (!(cfl > 0)) return fail(c, CFS_ERR_INVALID, "cfl must be positive");
     CFS_CUDA(c, cudaSetDevice(c->cfg.device));
-    CFS_CUDA(c, cudaMemsetAsync(c->wmax, 0, sizeof(unsigned long long), c->stream));
     CFS_CUDA(c, cfs::launch_wmax(c->L.elem_bytes, c->S[c->cur], c->L, c->has_types ? c->types_d : nullptr, c->cfg.gamma,
                                  c->dx, c->dy, c->wmax, c->stream));
-    unsigned long long bits = 0;
-    CFS_CUDA(c, cudaMemcpyAsync(&bits, c->wmax, sizeof(bits), cudaMemcpyDeviceToHost, c->stream));
+    CFS_CUDA(c, cfs::launch_results(c->results, nullptr, c->wmax, nullptr, c->stream));
     CFS_CUDA(c, cudaStreamSynchronize(c->stream));
     double m;
-    std::memcpy(&m, &bits, sizeof(m));
+    std::memcpy(&m, &c->results->wmax, sizeof(m));
     if (!(m > 0) || !std::isfinite(m))
         return fail(c, CFS_ERR_NUMERIC, "CFL reduction: a fluid cell is non-finite or every wave speed is 0");
     *dt = cfl / m;
@@ -903,14 +927,7 @@ int cfs_advance(cfs_ctx* c, int nsteps, double cfl, double dt, double* t_elapsed
     // one call of K steps takes), else reduced now
     const bool carry = hp.use_cfl && c->wmax_carry;
     if (carry) hp.wmax[0] = c->wmax_bits;
-    // (the previous advance ended with a stream synchronisation, so the pinned
-    // slot is free)
-    const cfs::DevParams* hp_src = &hp;
-    if (c->hp_pin) {
-        c->hp_pin[0] = hp;
-        hp_src = c->hp_pin;
-    }
-    CFS_CUDA(c, cudaMemcpyAsync(c->P, hp_src, sizeof(hp), cudaMemcpyHostToDevice, c->stream));
+    CFS_CUDA(c, cfs::launch_set_params(c->P, hp, c->stream));
     if (hp.use_cfl && !carry) {
         if (c->ib_n > 0) CFS_CUDA(c, cfs::launch_ib_fill(c->L.elem_bytes, ib_args(c, c->S[0]), c->stream));
         CFS_CUDA(c, cfs::launch_wmax(c->L.elem_bytes, c->S[0], c->L, c->has_types ? c->types_d : nullptr, c->cfg.gamma,
@@ -957,13 +974,11 @@ int cfs_advance(cfs_ctx* c, int nsteps, double cfl, double dt, double* t_elapsed
     for (int k = 0; k + 1 < nsteps; k += 2) CFS_CUDA(c, cudaGraphLaunch(c->graph2, c->stream));
     if (nsteps % 2 == 1) CFS_CUDA(c, cudaGraphLaunch(c->graph1, c->stream));
     cfs::DevParams out{};
-    CFS_CUDA(c, cudaMemcpyAsync(c->hp_pin ? c->hp_pin + 1 : &out, c->P, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
-    CFS_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (c->hp_pin) out = c->hp_pin[1];
+    const int rc_flags = wait_results(c, &out);
     if (t_elapsed) *t_elapsed = out.t;
     if (dt_last) *dt_last = out.dt_last;
     c->steps_done += static_cast<unsigned int>(nsteps);
-    if (const int rc = check_device_errors(c); rc != CFS_OK) return rc;
+    if (rc_flags != CFS_OK) return rc_flags;
     if (nsteps > 0) c->wmax_carry = false;
     if (nsteps > 0 && (!(out.dt_last > 0) || !std::isfinite(out.dt_last)))
         return fail(c, CFS_ERR_NUMERIC, "time step became non-finite or non-positive");
@@ -992,7 +1007,7 @@ int cfs_steps_begin(cfs_ctx* c, double cfl, double dt) {
     hp.seed[0] = hp.seed[1] = c->steps_done;
     const bool carry = hp.use_cfl && c->wmax_carry;
     if (carry) hp.wmax[0] = c->wmax_bits;
-    CFS_CUDA(c, cudaMemcpyAsync(c->P, &hp, sizeof(hp), cudaMemcpyHostToDevice, c->stream));
+    CFS_CUDA(c, cfs::launch_set_params(c->P, hp, c->stream));
     if (hp.use_cfl && !carry) {
         if (c->ib_n > 0) CFS_CUDA(c, cfs::launch_ib_fill(c->L.elem_bytes, ib_args(c, c->S[c->cur]), c->stream));
         CFS_CUDA(c, cfs::launch_wmax(c->L.elem_bytes, c->S[c->cur], c->L, c->has_types ? c->types_d : nullptr, c->cfg.gamma,
@@ -1080,10 +1095,9 @@ int cfs_steps_end(cfs_ctx* c, double* t_elapsed, double* dt_last) {
     if (c->next_stage != 0) return fail(c, CFS_ERR_STATE, "a step is in progress (stage sequence not at stage 0)");
     CFS_CUDA(c, cudaSetDevice(c->cfg.device));
     cfs::DevParams out{};
-    CFS_CUDA(c, cudaMemcpyAsync(&out, c->P, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
-    CFS_CUDA(c, cudaStreamSynchronize(c->stream));
+    const int rc_flags = wait_results(c, &out);
     c->in_steps = false;
-    if (const int rc = check_device_errors(c); rc != CFS_OK) return rc;
+    if (rc_flags != CFS_OK) return rc_flags;
     if (t_elapsed) *t_elapsed = out.t;
     if (dt_last) *dt_last = out.dt_last;
     if (out.t > 0 && (!(out.dt_last > 0) || !std::isfinite(out.dt_last)))
@@ -1099,8 +1113,7 @@ int cfs_steps_end(cfs_ctx* c, double* t_elapsed, double* dt_last) {
 int cfs_synchronize(cfs_ctx* c) {
     if (!c) return fail(c, CFS_ERR_INVALID, "null context");
     CFS_CUDA(c, cudaSetDevice(c->cfg.device));
-    CFS_CUDA(c, cudaStreamSynchronize(c->stream));
-    return check_device_errors(c);
+    return wait_results(c, nullptr);
 }
 
 void* cfs_get_stream(cfs_ctx* c) { return c ? static_cast<void*>(c->stream) : nullptr; }

@@ -147,6 +147,11 @@ void* state_buf(const cfs_batch* b, const BatchCase& c, int k) {
     return b->arena + c.state_off + static_cast<size_t>(k) * static_cast<size_t>(c.L.bytes());
 }
 
+cudaError_t fill_ghosts(cfs_batch* b, const BatchCase& c) {
+    void* const U[3] = {state_buf(b, c, 0), state_buf(b, c, 1), state_buf(b, c, 2)};
+    return cfs::launch_ghost_fill(b->elem, U, c.L, c.sides, b->stream);
+}
+
 // Host images of the per-case stage and fill arguments (device copies in
 // dargs / dib); rebuilt when storage offsets change.
 int upload_args(cfs_batch* b) {
@@ -499,10 +504,8 @@ int cfs_batch_create(const cfs_config* common, int ncases, const cfs_case* cases
          cudaMemset(b->P, 0, sizeof(cfs::DevParams) * ncases) == cudaSuccess;
     if (!ok) return bail(CFS_ERR_CUDA, "batch upload failed");
     for (int ci = 0; ci < ncases; ++ci)
-        for (int k = 0; k < 3; ++k)
-            if (cfs::launch_ghost_fill(b->elem, state_buf(b, b->cases[ci], k), b->cases[ci].L, b->cases[ci].sides,
-                                       b->stream) != cudaSuccess)
-                return bail(CFS_ERR_CUDA, "ghost fill failed");
+        if (fill_ghosts(b, b->cases[ci]) != cudaSuccess)
+            return bail(CFS_ERR_CUDA, "ghost fill failed");
     if (cudaStreamSynchronize(b->stream) != cudaSuccess || cudaGetLastError() != cudaSuccess)
         return bail(CFS_ERR_CUDA, "batch initialisation failed");
     *out = b;
@@ -528,7 +531,8 @@ int cfs_batch_set_state(cfs_batch* b, int ci, const double* U) {
         // FP32 storage offsets: the FP32-rounded means, summed on the device as
         // a single grid's (cfs_set_state) are
         double sums[kVars];
-        CFSB_CUDA(b, cfs::launch_plane_sums(b->staging, static_cast<long long>(n), b->sums, b->stream));
+        CFSB_CUDA(b, cfs::launch_plane_sums(b->staging, static_cast<long long>(n), b->sums,
+                                            b->sums + cfs::plane_sums_scratch_doubles() - kVars, b->stream));
         CFSB_CUDA(b, cudaMemcpyAsync(sums, b->sums + cfs::plane_sums_scratch_doubles() - kVars, sizeof(sums),
                                      cudaMemcpyDeviceToHost, b->stream));
         CFSB_CUDA(b, cudaStreamSynchronize(b->stream));
@@ -540,7 +544,7 @@ int cfs_batch_set_state(cfs_batch* b, int ci, const double* U) {
         }
     }
     CFSB_CUDA(b, cfs::launch_pack(b->elem, b->staging, state_buf(b, c, 0), c.L, b->stream));
-    for (int k = 0; k < 3; ++k) CFSB_CUDA(b, cfs::launch_ghost_fill(b->elem, state_buf(b, c, k), c.L, c.sides, b->stream));
+    CFSB_CUDA(b, fill_ghosts(b, c));
     CFSB_CUDA(b, cudaStreamSynchronize(b->stream));
     return CFS_OK;
 }

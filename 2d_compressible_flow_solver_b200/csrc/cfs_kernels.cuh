@@ -970,7 +970,8 @@ __device__ __forceinline__ bool ghost_value(const T* p, const Layout& L, const B
 }
 
 template <class T>
-__global__ void ghost_fill_kernel(T* U, const Layout L, BcSides sides) {
+__global__ void ghost_fill_kernel(T* U0, T* U1, T* U2, const Layout L, BcSides sides) {
+    T* const U = blockIdx.y == 0 ? U0 : blockIdx.y == 1 ? U1 : U2;
     const int per = (L.nx > L.ny ? L.nx : L.ny);
     const long long edge_items = 4LL * kGhost * per * kVars;
     const long long corner_items = 4LL * kGhost * kGhost * kVars;

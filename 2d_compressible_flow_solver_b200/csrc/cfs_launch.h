@@ -27,14 +27,22 @@ cudaError_t launch_batch_wmax(int elem_bytes, const StageArgs* args, int ncases,
 // Sums of the four planes of a device FP64 state [4][n], deterministic; the 4
 // sums land at scratch[plane_sums_scratch_doubles() - 4 ..].
 int plane_sums_scratch_doubles();
-cudaError_t launch_plane_sums(const double* U, long long n, double* scratch, cudaStream_t s);
+cudaError_t launch_plane_sums(const double* U, long long n, double* scratch, double* out4, cudaStream_t s);
+// The parameters of an advance to the device (P), and results to the host's
+// pinned memory (null sources are left out): one-thread kernels in the place of
+// copies of a few bytes, each of which took the copy engine and two to three
+// microseconds more.  wmax is set back to 0 behind the read.
+cudaError_t launch_set_params(DevParams* P, const DevParams& v, cudaStream_t s);
+cudaError_t launch_results(HostResults* out, const DevParams* P, unsigned long long* wmax, const unsigned int* err,
+                           cudaStream_t s);
 // Sums of the four planes over fluid cells, deterministic (fixed order);
 // scratch holds plane_sums_scratch_doubles() doubles, the 4 sums go to out.
 cudaError_t launch_totals(int elem_bytes, const void* U, const Layout& L, const uint8_t* types, double* scratch,
                           double* out, cudaStream_t s);
 cudaError_t launch_pack(int elem_bytes, const double* src, void* dst, const Layout& L, cudaStream_t s);
 cudaError_t launch_unpack(int elem_bytes, const void* src, double* dst, const Layout& L, cudaStream_t s);
-cudaError_t launch_ghost_fill(int elem_bytes, void* U, const Layout& L, const BcSides& sides, cudaStream_t s);
+// Ghost layers of the three state buffers, in one launch.
+cudaError_t launch_ghost_fill(int elem_bytes, void* const U[3], const Layout& L, const BcSides& sides, cudaStream_t s);
 cudaError_t launch_viscous(Prec p, const ViscArgs& a, cudaStream_t s);
 cudaError_t launch_weno_faces(Prec p, int n, const double* st, double* left, double* right, double g, double eps,
                               cudaStream_t s);

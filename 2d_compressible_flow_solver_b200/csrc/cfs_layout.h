@@ -77,6 +77,15 @@ struct DevParams {
     unsigned int seed[2];         // stochastic-rounding step counter, ping-pong per step
 };
 
+// What the host reads back after a wait, in pinned memory that the device
+// writes directly.
+struct HostResults {
+    DevParams params;             // cfs_advance
+    double sums[4];               // plane sums of an uploaded state
+    unsigned long long wmax;      // cfs_compute_dt
+    unsigned int err;             // device error flags
+};
+
 struct StageArgs {
     const void* in;        // state differentiated this stage (tile + halo reads)
     const void* u0;        // RK stage-0 copy (pointwise reads), stage >= 1

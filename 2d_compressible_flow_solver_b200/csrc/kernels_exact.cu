@@ -157,9 +157,9 @@ __global__ void plane_final_sums_kernel(const double* partial, double* out4) {
 
 int plane_sums_scratch_doubles() { return kVars * kSumBlocks + kVars; }
 
-cudaError_t launch_plane_sums(const double* U, long long n, double* scratch, cudaStream_t s) {
+cudaError_t launch_plane_sums(const double* U, long long n, double* scratch, double* out4, cudaStream_t s) {
     plane_partial_sums_kernel<<<dim3(kSumBlocks, kVars), kSumThreads, 0, s>>>(U, n, scratch);
-    plane_final_sums_kernel<<<1, 32, 0, s>>>(scratch, scratch + kVars * kSumBlocks);
+    plane_final_sums_kernel<<<1, 32, 0, s>>>(scratch, out4);
     return cudaGetLastError();
 }
 
@@ -188,11 +188,34 @@ cudaError_t launch_unpack(int elem_bytes, const void* src, double* dst, const La
     return cudaGetLastError();
 }
 
-cudaError_t launch_ghost_fill(int elem_bytes, void* U, const Layout& L, const BcSides& sides, cudaStream_t s) {
+__global__ void set_params_kernel(DevParams* P, const DevParams v) { *P = v; }
+
+__global__ void results_kernel(HostResults* out, const DevParams* P, unsigned long long* wmax, const unsigned int* err) {
+    after_previous();
+    if (P) out->params = *P;
+    if (wmax) {
+        out->wmax = *wmax;
+        *wmax = 0ull;
+    }
+    if (err) out->err = *err;
+}
+
+cudaError_t launch_set_params(DevParams* P, const DevParams& v, cudaStream_t s) {
+    set_params_kernel<<<1, 1, 0, s>>>(P, v);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_results(HostResults* out, const DevParams* P, unsigned long long* wmax, const unsigned int* err,
+                           cudaStream_t s) {
+    return launch_after(results_kernel, 1, 1, 0, s, out, P, wmax, err);
+}
+
+cudaError_t launch_ghost_fill(int elem_bytes, void* const U[3], const Layout& L, const BcSides& sides, cudaStream_t s) {
     const int per = L.nx > L.ny ? L.nx : L.ny;
     const int nt = 256, nb = flat_blocks(4LL * kGhost * per * kVars + 4LL * kGhost * kGhost * kVars, nt);
-    if (elem_bytes == 8) ghost_fill_kernel<double><<<nb, nt, 0, s>>>(static_cast<double*>(U), L, sides);
-    else ghost_fill_kernel<float><<<nb, nt, 0, s>>>(static_cast<float*>(U), L, sides);
+    const dim3 grid(nb, 3);
+    if (elem_bytes == 8) ghost_fill_kernel<<<grid, nt, 0, s>>>(static_cast<double*>(U[0]), static_cast<double*>(U[1]), static_cast<double*>(U[2]), L, sides);
+    else ghost_fill_kernel<<<grid, nt, 0, s>>>(static_cast<float*>(U[0]), static_cast<float*>(U[1]), static_cast<float*>(U[2]), L, sides);
     return cudaGetLastError();
 }
 
