@@ -119,6 +119,8 @@ struct StageArgs {
                            // (row_hi 0: up to nx); a decomposed grid updates its interior
                            // rows while the halo exchange is in flight, then its edge rows
     int rows;              // row march: rows of one warp's work item (0: the launcher chooses)
+    int long_chunks;       // row march: chunks of `rows` rows per segment; shorter ones of rows_short follow
+    int rows_short;
     unsigned int* err;     // device error flags (kErr* bits), set instead of waiting forever
     int has_tmaps;         // 1: tmap_in (and, stage >= 1, tmap_u0) hold encoded tensor maps
     // TMA load schedule: tensor maps (CUtensorMap) of the `in` and `u0` buffers,

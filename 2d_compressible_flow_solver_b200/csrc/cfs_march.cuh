@@ -729,7 +729,7 @@ __device__ __forceinline__ void y_part(const StageArgs& a, const UpdateCoefs& k,
 // instruction cache stalls every warp on instruction fetch, whatever the share
 // of the rare code actually executed.
 template <class Pol, int kWarps, int kLoad, int kFeat>
-__device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, int rows,
+__device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int i0, int i1, bool first,
                                            typename Pol::C (&rbuf)[kWarps][36][kVars],
                                            typename Pol::T* ring, int wid, unsigned long long* bars = nullptr,
                                            unsigned* phase = nullptr) {
@@ -745,8 +745,6 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
     const Layout& L = a.L;
     const int lane = threadIdx.x & 31;
     const int j0 = seg * kSeg;
-    const int i0 = stage_row_lo(a) + by * rows;
-    const int i1 = min(i0 + rows, stage_row_hi(a));
     const int j = j0 - 1 + lane;                 // this lane's column
     const bool col_ok = j <= L.ny + kGhost - 1;  // inside the padded row
     const bool owner = lane >= 1 && lane <= kSeg && j < L.ny;  // updates cells of this column
@@ -760,7 +758,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int by, 
     const C* const bfl = static_cast<const C*>(a.bflux);
     const uint8_t* const flags = kEdge ? a.cflags : nullptr;
     const T* const rv_in = kExtra ? static_cast<const T*>(a.rv) : nullptr;
-    if (a.P && a.first_stage && seg == 0 && by == 0 && lane == 0) begin_step(a, uc.dt);
+    if (a.P && a.first_stage && first && lane == 0) begin_step(a, uc.dt);
     const bool active_warp = j0 < L.ny;  // uniform per warp
 
     auto load_row = [&](int r, C out[kVars]) {
@@ -1085,22 +1083,27 @@ __device__ __forceinline__ void init_ring_bars(unsigned long long (&bars)[kWarps
 
 template <class Pol, int kRows, int kWarps, int kMinBlocks, int kLoad, int kFeat>
 __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) march_kernel(const __grid_constant__ StageArgs a) {
-    // rows of this launch's work items: chosen by the launcher (a.rows), or the variant's
-    const int rows = a.rows > 0 ? a.rows : kRows;
     // warps numbered over (segment, row chunk), segments fastest, so no block
     // carries idle warps when the segments of a row are not a multiple of its
-    // warps; a warp past the last item runs an empty one
-    const int nseg = (a.L.ny + kSeg - 1) / kSeg;
-    const long long nitems =
-        static_cast<long long>(nseg) * ((stage_row_hi(a) - stage_row_lo(a) + rows - 1) / rows);
+    // warps; a warp past the last item runs an empty one.  The long chunks come
+    // first, the short ones behind them fill the launch's end.
     // (the warp index taken from lane 0, so that the compiler knows the item's
     // rows and columns to be the same in all lanes: the row tests' branches need
     // no convergence code.  685 -> 670 instructions per cell-stage in FP32, the
     // 4096^2 step 1,384 -> 1,356 us, 2048^2 FP64 689 -> 666)
+    const int nseg = (a.L.ny + kSeg - 1) / kSeg;
     const int wid = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
     const long long gw = static_cast<long long>(blockIdx.x) * kWarps + wid;
-    const int seg = gw < nitems ? static_cast<int>(gw % nseg) : nseg;
-    const int by = gw < nitems ? static_cast<int>(gw / nseg) : 0;
+    const int chunk = static_cast<int>(gw / nseg), lo = stage_row_lo(a), hi = stage_row_hi(a);
+    const bool is_long = chunk < a.long_chunks;
+    const long long at = is_long ? static_cast<long long>(chunk) * a.rows
+                                 : static_cast<long long>(a.long_chunks) * a.rows +
+                                       static_cast<long long>(chunk - a.long_chunks) * a.rows_short;
+    const bool item = at < hi - lo;
+    const int seg = item ? static_cast<int>(gw % nseg) : nseg;
+    const int i0 = item ? lo + static_cast<int>(at) : lo;
+    const int i1 = min(i0 + (is_long ? a.rows : a.rows_short), hi);
+    const bool first = gw == 0;
     after_previous();
     // (the ring forms use no row buffer)
     __shared__ __align__(16) typename Pol::C rbuf[kLoad >= 3 ? 1 : kWarps][36][kVars];
@@ -1115,26 +1118,26 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) march_kernel(const __
         unsigned phase = 0u;
         if constexpr (sizeof(typename Pol::T) == 4) {
             __shared__ __align__(128) typename Pol::T ring[kWarps * ring_words<typename Pol::T, kLoad>()];
-            march_item<Pol, kWarps, kLoad, kFeat>(a, seg, by, rows, reinterpret_cast<RB>(rbuf), ring, wid,
+            march_item<Pol, kWarps, kLoad, kFeat>(a, seg, i0, i1, first, reinterpret_cast<RB>(rbuf), ring, wid,
                                                   bars[wid], &phase);
         } else {
             // FP64 ring: dynamic shared memory, sized at launch
             extern __shared__ __align__(128) unsigned char march_dyn_smem[];
-            march_item<Pol, kWarps, kLoad, kFeat>(a, seg, by, rows, reinterpret_cast<RB>(rbuf),
+            march_item<Pol, kWarps, kLoad, kFeat>(a, seg, i0, i1, first, reinterpret_cast<RB>(rbuf),
                                                   reinterpret_cast<typename Pol::T*>(march_dyn_smem), wid, bars[wid],
                                                   &phase);
         }
     } else if constexpr (kLoad == 3 && sizeof(typename Pol::T) == 4) {
         __shared__ __align__(128) typename Pol::T ring[kWarps * ring_words<typename Pol::T, kLoad>()];
-        march_item<Pol, kWarps, kLoad, kFeat>(a, seg, by, rows, reinterpret_cast<RB>(rbuf), ring, wid);
+        march_item<Pol, kWarps, kLoad, kFeat>(a, seg, i0, i1, first, reinterpret_cast<RB>(rbuf), ring, wid);
     } else if constexpr (kLoad == 3) {
         // FP64 ring: kWarps * ring_words<double, 3>() doubles (36.9 KB for 4
         // warps); dynamic shared memory, sized at launch
         extern __shared__ __align__(128) unsigned char march_dyn_smem[];
-        march_item<Pol, kWarps, kLoad, kFeat>(a, seg, by, rows, reinterpret_cast<RB>(rbuf),
+        march_item<Pol, kWarps, kLoad, kFeat>(a, seg, i0, i1, first, reinterpret_cast<RB>(rbuf),
                                               reinterpret_cast<typename Pol::T*>(march_dyn_smem), wid);
     } else {
-        march_item<Pol, kWarps, kLoad, kFeat>(a, seg, by, rows, rbuf, nullptr, wid);
+        march_item<Pol, kWarps, kLoad, kFeat>(a, seg, i0, i1, first, rbuf, nullptr, wid);
     }
 }
 
@@ -1171,7 +1174,8 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks)
         const int c = unit_case[w], lu = unit_local[w];
         const int ns = case_nseg[c];
         const StageArgs a = args[c];
-        march_item<Pol, 1, kLoad, kFeat>(a, lu % ns, lu / ns, case_rows[c], wbuf, kRing ? ring + wid * ring_words<typename Pol::T, kLoad>() : nullptr, 0);
+        const int rows = case_rows[c], i0 = lu / ns * rows;
+        march_item<Pol, 1, kLoad, kFeat>(a, lu % ns, i0, min(i0 + rows, a.L.nx), lu == 0, wbuf, kRing ? ring + wid * ring_words<typename Pol::T, kLoad>() : nullptr, 0);
     }
 }
 

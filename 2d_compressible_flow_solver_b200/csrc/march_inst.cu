@@ -53,12 +53,21 @@ cudaError_t launch_march(const StageArgs& a_in, cudaStream_t s) {
     }
     static ResidentCache cache;
     const long long slots = resident_blocks(cache, march_kernel<Pol, R, W, B, Ld, F>, 32 * W, dyn);
-    const int rows = a.rows > 0 ? a.rows : slots > 0 ? choose_rows(nseg, W, nrows, slots) : R;  // (a failed query: fixed rows)
-    // one warp per (segment, row chunk), segments fastest
-    const long long items = static_cast<long long>(nseg) * ((nrows + rows - 1) / rows);
-    const dim3 grid(static_cast<unsigned>((items + W - 1) / W));
     StageArgs b = a;
-    b.rows = rows;
+    if (a.rows > 0 || slots <= 0) {  // fixed rows (also where the query of the slots failed)
+        b.rows = b.rows_short = a.rows > 0 ? a.rows : R;
+        b.long_chunks = (nrows + b.rows - 1) / b.rows;
+    } else {
+        const RowChunks c = choose_chunks(nseg, W, nrows, slots);
+        b.rows = c.rows;
+        b.long_chunks = c.long_chunks;
+        b.rows_short = c.rows_short;
+    }
+    const int covered = b.long_chunks * b.rows;
+    const int chunks = b.long_chunks + (covered < nrows ? (nrows - covered + b.rows_short - 1) / b.rows_short : 0);
+    // one warp per (segment, row chunk), segments fastest
+    const long long items = static_cast<long long>(nseg) * chunks;
+    const dim3 grid(static_cast<unsigned>((items + W - 1) / W));
     // A launch of more blocks than fit at once starts before the one ahead of it
     // ends (launch_after).  A smaller one waits for it: its blocks would go to
     // whichever SMs have room, two and three to some, and the stage lasts as long
