@@ -15,8 +15,8 @@ trying the candidate rows with the others fixed, writing
 ``batch_rows[precision] = {"rows": {bucket: rows}, ...}`` beside the variant
 table.  (Uniform batches of one size prefer shorter units than the same sizes
 among larger cases do, so the sweep runs on the mixed workload.)
-``batch_rows_for(precision, nx, ny)`` reads it back: the Batch wrapper gives
-every case whose rows are not set the rows of its bucket.
+``batch_rows_for(precision, nx, ny)`` reads it back, for a caller that fixes
+``rows`` per case; units that the library cuts itself (``rows`` = 0) are faster.
 
 Usage (on a GPU): ``python -m 2d_compressible_flow_solver_b200.autotune`` is not
 importable by name, so run ``python 2d_compressible_flow_solver_b200/autotune.py

@@ -27,7 +27,7 @@ struct BatchCase {
     double dx = 0, dy = 0;
     size_t state_off = 0;   // bytes from the arena start to S0 (S1, S2 follow)
     long long types_off = -1;
-    int rows = 32, nseg = 0, items_y = 0;  // row chunk, 30-column segments, row chunks
+    int nseg = 0;  // 30-column segments
     std::vector<uint8_t> types;
     std::vector<uint8_t> lowo;   // CFS_POSITIVITY_BODY face flags, [nx+1][ny+1]
     long long lowo_off = -1;
@@ -44,7 +44,7 @@ struct BatchCase {
 // neither physical sides nor a body runs no edge code.
 struct FeatureGroup {
     int feat = 0;
-    int first = 0, count = 0;  // range of the group's items in item_case / item_local
+    int first = 0, count = 0;  // range of the group's items in units
 };
 
 }  // namespace
@@ -76,10 +76,7 @@ struct cfs_batch {
     cfs::StageArgs* dargs = nullptr;  // [parity][stage][case]
     cfs::IbArgs* dib = nullptr;       // [input buffer][case]
     int total_items = 0;
-    int* item_case = nullptr;
-    int* item_local = nullptr;
-    int* case_rows = nullptr;
-    int* case_nseg = nullptr;
+    cfs::BatchUnit* units = nullptr;
     unsigned int* counters = nullptr;  // [parity][stage][group] (cfs::kBatchCounters)
     double* staging = nullptr;
     double* sums = nullptr;  // plane sums of an uploaded case state (FP32 storage offsets)
@@ -118,29 +115,43 @@ int stages_of(int rk) { return rk == CFS_RK_TVD2 ? 2 : 3; }
 // FP64 bit pattern of +infinity: the CFL maximum of a state with a non-finite fluid cell
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
 
-// Rows of a work unit where a case sets none: the chunk of the single-grid
-// launches (choose_rows), over the units of all cases and the `warps` resident
-// ones -- a unit of R rows costs about R + 2, and a stage lasts about
-// (R + 2) (units / warps + 1/2).  A large batch gets long units (71 rows on
-// 512 uneven cases of 64 .. 768 cells, where a sweep had found 64 to 96 best),
-// a small one short ones, or most warps would find no unit.  SSP3 steps with
-// 64 rows (the default before) and these, FP32 / FP64: 4 cases to 256 cells
-// 440 -> 66 / 694 -> 93 us, 24 to 512 562 -> 306 / 949 -> 491, 48 to 768
-// 1,123 -> 1,020 / 1,917 -> 1,697; within 2 % of the best of a sweep of 2 ..
-// 96 rows from 8 to 256 cases.
-int default_rows(const std::vector<BatchCase>& cases, long long warps) {
-    int best_r = cfs::kBatchMaxRows;
-    long long best_cost = -1;
-    for (int r = 1; r <= cfs::kBatchMaxRows; ++r) {
-        long long units = 0;
-        for (const BatchCase& c : cases) units += static_cast<long long>(c.nseg) * ((c.desc.nx + r - 1) / r);
-        const long long cost = static_cast<long long>(r + 2) * (2 * units + warps);
-        if (best_cost < 0 || cost <= best_cost) {
-            best_cost = cost;
-            best_r = r;
+// Work units of one launch: the cases order[0 .. n), the largest first.  The
+// rows of a case that sets none are cut with the work that is left: a unit gets
+// 0.7 of what remains for each of the `warps` resident ones (96 rows at most),
+// down to 0.8 sqrt(rows per warp).  Long units first repeat few rows (each
+// repeats 2), and the warps, which draw their units from one counter, end
+// together on the short ones.  Against equal units of the length that balances
+// the two (16 to 30 rows on these batches), SSP3 steps FP32 / FP64: 4 cases to
+// 256 cells 52.8 -> 47.8 / 82 -> 70 us, 24 to 512 262 -> 252 / 470 -> 454, 48 to
+// 768 890 -> 846 / 1,678 -> 1,620, 128 to 768 2,144 -> 2,054 / 4,122 -> 3,958; 8
+// to 768 the same.  Shares of 0.25 .. 0.9 and shortest units of 0.2 .. 1.0
+// sqrt(rows per warp) were swept: 0.5 loses 6 % on the batch of 24, 0.75 3 %
+// on the one of 48.
+void append_units(const std::vector<BatchCase>& cases, const int* order, int n, long long warps,
+                  std::vector<cfs::BatchUnit>& units) {
+    double total = 0;  // rows of segments that the library cuts
+    for (int k = 0; k < n; ++k) {
+        const BatchCase& c = cases[order[k]];
+        if (c.desc.rows <= 0) total += static_cast<double>(c.nseg) * c.desc.nx;
+    }
+    const double per_warp = total / static_cast<double>(warps);
+    const int r_min = std::max(2, static_cast<int>(0.8 * std::sqrt(per_warp) + 0.5));
+    double left = total;
+    for (int k = 0; k < n; ++k) {
+        const int ci = order[k];
+        const BatchCase& c = cases[ci];
+        for (int i0 = 0; i0 < c.desc.nx;) {
+            int rows = c.desc.rows;
+            if (rows <= 0) {
+                const double share = std::min(0.7 * left / static_cast<double>(warps), double(cfs::kBatchMaxRows));
+                rows = std::max(r_min, static_cast<int>(share + 0.5));
+                left -= static_cast<double>(c.nseg) * std::min(rows, c.desc.nx - i0);
+            }
+            const int i1 = i0 + std::min(rows, c.desc.nx - i0);
+            for (int seg = 0; seg < c.nseg; ++seg) units.push_back({ci, seg, i0, i1});
+            i0 = i1;
         }
     }
-    return best_r;
 }
 
 void* state_buf(const cfs_batch* b, const BatchCase& c, int k) {
@@ -246,8 +257,7 @@ int enqueue_batch_step(cfs_batch* b, int parity) {
         for (size_t g = 0; g < b->groups.size(); ++g) {
             const FeatureGroup& fg = b->groups[g];
             CFSB_CUDA(b, cfs::launch_batch_stage(b->prec, b->dargs + static_cast<size_t>(slot) * b->n,
-                                                 b->item_case + fg.first, b->item_local + fg.first, b->case_rows,
-                                                 b->case_nseg, fg.count, b->counters, slot * cfs::kBatchMaxGroups + static_cast<int>(g),
+                                                 b->units + fg.first, fg.count, b->counters, slot * cfs::kBatchMaxGroups + static_cast<int>(g),
                                                  b->grid, fg.feat, scheme, b->stream));
         }
     }
@@ -279,10 +289,7 @@ int cfs_batch_destroy(cfs_batch* b) {
     cudaFree(b->P);
     cudaFree(b->dargs);
     cudaFree(b->dib);
-    cudaFree(b->item_case);
-    cudaFree(b->item_local);
-    cudaFree(b->case_rows);
-    cudaFree(b->case_nseg);
+    cudaFree(b->units);
     cudaFree(b->counters);
     cudaFree(b->staging);
     cudaFree(b->sums);
@@ -406,16 +413,11 @@ int cfs_batch_create(const cfs_config* common, int ncases, const cfs_case* cases
     }
     b->total_ig = static_cast<int>(h_cell.size());
 
-    // --- rows of a work unit, for the cases that leave them to the library
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, common->device) != cudaSuccess || sms <= 0)
         return bail(CFS_ERR_CUDA, "SM count query failed");
     b->grid = sms * cfs::batch_blocks_per_sm(b->prec);
-    const int rows = default_rows(b->cases, static_cast<long long>(b->grid) * cfs::kBatchWarps);
-    for (BatchCase& c : b->cases) {
-        c.rows = c.desc.rows > 0 ? c.desc.rows : rows;
-        c.items_y = (c.desc.nx + c.rows - 1) / c.rows;
-    }
+    const long long warps = static_cast<long long>(b->grid) * cfs::kBatchWarps;
 
     // --- features per case: edge code where a case has a physical side or
     // a body, positivity code as the batch's mode asks
@@ -435,26 +437,19 @@ int cfs_batch_create(const cfs_config* common, int ncases, const cfs_case* cases
                static_cast<long long>(b->cases[y].desc.nx) * b->cases[y].desc.ny;
     });
     // one work unit per (segment, row chunk): a warp's share of a stage
-    std::vector<int> it_case, it_local, c_rows(ncases), c_ix(ncases);
-    for (int ci : order) {
-        const BatchCase& c = b->cases[ci];
-        if (b->groups.empty() || b->groups.back().feat != c.feat) {
-            FeatureGroup g;
-            g.feat = c.feat;
-            g.first = static_cast<int>(it_case.size());
-            b->groups.push_back(g);
-        }
-        for (int li = 0; li < c.nseg * c.items_y; ++li) {
-            it_case.push_back(ci);
-            it_local.push_back(li);
-        }
-        b->groups.back().count = static_cast<int>(it_case.size()) - b->groups.back().first;
+    std::vector<cfs::BatchUnit> units;
+    for (int first = 0; first < ncases;) {
+        int end = first;
+        while (end < ncases && b->cases[order[end]].feat == b->cases[order[first]].feat) ++end;
+        FeatureGroup g;
+        g.feat = b->cases[order[first]].feat;
+        g.first = static_cast<int>(units.size());
+        append_units(b->cases, order.data() + first, end - first, warps, units);
+        g.count = static_cast<int>(units.size()) - g.first;
+        b->groups.push_back(g);
+        first = end;
     }
-    for (int ci = 0; ci < ncases; ++ci) {
-        c_rows[ci] = b->cases[ci].rows;
-        c_ix[ci] = b->cases[ci].nseg;
-    }
-    b->total_items = static_cast<int>(it_case.size());
+    b->total_items = static_cast<int>(units.size());
 
     // --- device allocations
     auto dalloc = [&](void** p, size_t bytes) { return bytes == 0 || cudaMalloc(p, bytes) == cudaSuccess; };
@@ -472,10 +467,7 @@ int cfs_batch_create(const cfs_config* common, int ncases, const cfs_case* cases
         !dalloc(reinterpret_cast<void**>(&b->P), sizeof(cfs::DevParams) * ncases) ||
         !dalloc(reinterpret_cast<void**>(&b->dargs), sizeof(cfs::StageArgs) * 6 * ncases) ||
         !dalloc(reinterpret_cast<void**>(&b->dib), sizeof(cfs::IbArgs) * 3 * ncases) ||
-        !dalloc(reinterpret_cast<void**>(&b->item_case), sizeof(int) * it_case.size()) ||
-        !dalloc(reinterpret_cast<void**>(&b->item_local), sizeof(int) * it_local.size()) ||
-        !dalloc(reinterpret_cast<void**>(&b->case_rows), sizeof(int) * ncases) ||
-        !dalloc(reinterpret_cast<void**>(&b->case_nseg), sizeof(int) * ncases) ||
+        !dalloc(reinterpret_cast<void**>(&b->units), sizeof(cfs::BatchUnit) * units.size()) ||
         !dalloc(reinterpret_cast<void**>(&b->counters), sizeof(unsigned int) * cfs::kBatchCounters) ||
         !dalloc(reinterpret_cast<void**>(&b->staging), sizeof(double) * kVars * max_cells) ||
         !dalloc(reinterpret_cast<void**>(&b->sums), sizeof(double) * cfs::plane_sums_scratch_doubles()))
@@ -497,9 +489,7 @@ int cfs_batch_create(const cfs_config* common, int ncases, const cfs_case* cases
          h2d(b->ib_fac, h_fac.data(), sizeof(double) * h_fac.size()) &&
          h2d(b->ig_case, h_igc.data(), sizeof(int) * h_igc.size()) &&
          h2d(b->ig_local, h_igl.data(), sizeof(int) * h_igl.size()) &&
-         h2d(b->item_case, it_case.data(), sizeof(int) * it_case.size()) &&
-         h2d(b->item_local, it_local.data(), sizeof(int) * it_local.size()) &&
-         h2d(b->case_rows, c_rows.data(), sizeof(int) * ncases) && h2d(b->case_nseg, c_ix.data(), sizeof(int) * ncases) &&
+         h2d(b->units, units.data(), sizeof(cfs::BatchUnit) * units.size()) &&
          cudaMemset(b->counters, 0, sizeof(unsigned int) * cfs::kBatchCounters) == cudaSuccess &&
          cudaMemset(b->P, 0, sizeof(cfs::DevParams) * ncases) == cudaSuccess;
     if (!ok) return bail(CFS_ERR_CUDA, "batch upload failed");

@@ -162,11 +162,9 @@ constexpr int kBatchMinBlocksF64 = 4;
 // SM): the uneven 512-case batch 3,230 against 2,938 Mcell-steps/s without it
 // (the earlier ring that also held U^0 rows allowed 3 blocks and lost, 2,775).
 constexpr int kBatchLoadF64 = 3;
-// Longest batch work unit the library chooses by itself (cfs_case.rows = 0;
-// the rule is default_rows, cfs_batch.cpp): longer ones gain nothing (the
-// uneven 512-case batch: FP32 8,408 / 8,651 / 8,763 / 8,838 / 8,854 and FP64
-// 5,019 / 5,217 / 5,294 / 5,340 / 5,341 Mcell-steps/s at 16 / 24 / 32 / 48 /
-// 64 rows).
+// Longest batch work unit the library cuts by itself (append_units): longer
+// ones gain nothing (128 uneven cases to 768 cells at 128 / 96 / 64 rows, FP32
+// 2,131 / 2,066 / 2,069 us a step).
 constexpr int kBatchMaxRows = 96;
 // Work-unit counters of a batch, [parity][stage][feature group]: the group
 // launches of a stage count their own up from 0 and put every counter of the
@@ -174,8 +172,7 @@ constexpr int kBatchMaxRows = 96;
 // needs a clearing launch.
 constexpr int kBatchMaxGroups = 4;  // the feature sets a batch launches: 0, Pos, Edge, Edge | Pos
 constexpr int kBatchCounters = 2 * 3 * kBatchMaxGroups;
-cudaError_t launch_batch_stage(Prec p, const StageArgs* args, const int* item_case, const int* item_local,
-                               const int* case_rows, const int* case_nseg, int total, unsigned int* counters,
+cudaError_t launch_batch_stage(Prec p, const StageArgs* args, const BatchUnit* units, int total, unsigned int* counters,
                                int slot, int grid, int feat, int scheme,
                                cudaStream_t s);  // feat: kFeatPos | kFeatEdge bits; scheme: known_scheme
 // The same for a batch: the immersed-ghost cells of every case (total; may be

@@ -221,4 +221,9 @@ struct IbArgs {
     const int* perm;       // [4n] reference pivot order
 };
 
+// A work unit of a batched stage: rows [i0, i1) of one 30-column segment of a case.
+struct alignas(16) BatchUnit {
+    int ci, seg, i0, i1;
+};
+
 }  // namespace cfs

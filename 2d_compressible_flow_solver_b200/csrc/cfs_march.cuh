@@ -1149,9 +1149,8 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) march_kernel(const __
 // buffers, dt slot); rows[c] is its row chunk, nseg[c] its segment count.
 template <class Pol, int kWarps, int kMinBlocks, int kLoad, int kFeat>
 __global__ void __launch_bounds__(32 * kWarps, kMinBlocks)
-    batch_march_kernel(const StageArgs* __restrict__ args, const int* __restrict__ unit_case,
-                       const int* __restrict__ unit_local, const int* __restrict__ case_rows,
-                       const int* __restrict__ case_nseg, int total, unsigned int* counters, int slot) {
+    batch_march_kernel(const StageArgs* __restrict__ args, const BatchUnit* __restrict__ units, int total,
+                       unsigned int* counters, int slot) {
     using C = typename Pol::C;
     constexpr bool kRing = kLoad == 3;
     __shared__ __align__(16) C rbuf[kRing ? 1 : kWarps][36][kVars];  // (the ring forms use no row buffer)
@@ -1171,11 +1170,9 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks)
         if (lane == 0) w = atomicAdd(counter, 1u);
         w = __shfl_sync(0xffffffffu, w, 0);
         if (w >= static_cast<unsigned int>(total)) break;
-        const int c = unit_case[w], lu = unit_local[w];
-        const int ns = case_nseg[c];
-        const StageArgs a = args[c];
-        const int rows = case_rows[c], i0 = lu / ns * rows;
-        march_item<Pol, 1, kLoad, kFeat>(a, lu % ns, i0, min(i0 + rows, a.L.nx), lu == 0, wbuf, kRing ? ring + wid * ring_words<typename Pol::T, kLoad>() : nullptr, 0);
+        const int4 u = __ldg(reinterpret_cast<const int4*>(units) + w);  // a BatchUnit
+        const StageArgs a = args[u.x];
+        march_item<Pol, 1, kLoad, kFeat>(a, u.y, u.z, u.w, u.y == 0 && u.z == 0, wbuf, kRing ? ring + wid * ring_words<typename Pol::T, kLoad>() : nullptr, 0);
     }
 }
 

@@ -89,14 +89,13 @@ cudaError_t allow_dyn(Kernel k, size_t bytes) {
 }
 
 template <class Pol, int kMinBlocks, int kLoad, int kFeat>
-cudaError_t launch_batch_kernel(const StageArgs* args, const int* item_case, const int* item_local, const int* case_rows,
-                                const int* case_nseg, int total, unsigned int* counters, int slot, int grid,
+cudaError_t launch_batch_kernel(const StageArgs* args, const BatchUnit* units, int total, unsigned int* counters, int slot, int grid,
                                 cudaStream_t s) {
     constexpr size_t dyn = batch_dyn_bytes<Pol, kLoad>();
     const cudaError_t e = allow_dyn(batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeat>, dyn);
     if (e != cudaSuccess) return e;
     return launch_after(batch_march_kernel<Pol, kBatchWarps, kMinBlocks, kLoad, kFeat>, grid, 32 * kBatchWarps, dyn, s, args,
-                        item_case, item_local, case_rows, case_nseg, total, counters, slot);
+                        units, total, counters, slot);
 }
 
 template <class Pol, int kMinBlocks, int kLoad, int kScheme, class... Args>
@@ -121,15 +120,14 @@ cudaError_t launch_batch_scheme(int scheme, int feat, Args... args) {
     }
 }
 
-cudaError_t launch_batch_stage(Prec p, const StageArgs* args, const int* item_case, const int* item_local,
-                               const int* case_rows, const int* case_nseg, int total, unsigned int* counters,
+cudaError_t launch_batch_stage(Prec p, const StageArgs* args, const BatchUnit* units, int total, unsigned int* counters,
                                int slot, int grid, int feat, int scheme, cudaStream_t s) {
     if (total <= 0) return cudaSuccess;
     if (p == kF32Mixed)
         return launch_batch_scheme<PolF32, kBatchMinBlocksF32, kBatchLoadF32>(
-            scheme, feat, args, item_case, item_local, case_rows, case_nseg, total, counters, slot, grid, s);
+            scheme, feat, args, units, total, counters, slot, grid, s);
     return launch_batch_scheme<PolF64, kBatchMinBlocksF64, kBatchLoadF64>(
-        scheme, feat, args, item_case, item_local, case_rows, case_nseg, total, counters, slot, grid, s);
+        scheme, feat, args, units, total, counters, slot, grid, s);
 }
 
 int batch_blocks_per_sm(Prec p) {
