@@ -370,6 +370,18 @@ __device__ __forceinline__ void fix_states(bool lowL, bool lowR, const typename 
     }
 }
 
+// The same for the 32 lanes of a warp together (all of them call): flags f, of
+// which lowL and lowR mark the low-order faces.  One test over both states and
+// a branch that the warp takes as one.
+template <class Pol>
+__device__ __forceinline__ void fix_states_warp(unsigned int f, unsigned int lowL, unsigned int lowR,
+                                                const typename Pol::C c[kVars], double g, Face5<typename Pol::C>& L,
+                                                Face5<typename Pol::C>& R) {
+    using C = typename Pol::C;
+    const bool ok = (L.r > C(0)) & (L.p > C(0)) & (R.r > C(0)) & (R.p > C(0)) & !(f & (lowL | lowR));
+    if (!__all_sync(0xffffffffu, ok)) fix_states<Pol>(f & lowL, f & lowR, c, g, L, R);
+}
+
 // The same fallback on the two states of a physical boundary face, each taking
 // the value of the cell on its side (cl left of the face, cr right of it).
 template <class Pol>
@@ -669,7 +681,7 @@ __device__ __forceinline__ void y_part(const StageArgs& a, const UpdateCoefs& k,
     if constexpr ((kFeat & kFeatPos) != 0) {
         C cc[kVars];
         full(st[2], cc);
-        fix_states<Pol>(f_r & kCellLowYhi, f_r & kCellLowYlo, cc, g, Ly, Ry);
+        fix_states_warp<Pol>(f_r, kCellLowYhi, kCellLowYlo, cc, g, Ly, Ry);
     }
     // right state of the cell above (lane + 1)
     Face5<C> Rn;
@@ -753,7 +765,8 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int i0, 
     const double g = a.gamma;
     const UpdateCoefs uc = update_coefs<Pol, kFeat>(a);
     // physical boundary faces: the cell's own flux (transmissive) or a precomputed one (Dirichlet)
-    const bool lo_x = kEdge && physical_side(a, 0), hi_x = kEdge && physical_side(a, 1);
+    // rows below which a physical x-face lies (-2: none)
+    const int wall_lo = kEdge && physical_side(a, 0) ? 0 : -2, wall_hi = kEdge && physical_side(a, 1) ? L.nx : -2;
     const bool lo_y = kEdge && physical_side(a, 2), hi_y = kEdge && physical_side(a, 3);
     const C* const bfl = static_cast<const C*>(a.bflux);
     const uint8_t* const flags = kEdge ? a.cflags : nullptr;
@@ -787,12 +800,16 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int i0, 
             }
         }
     };
-    // Flag byte of cell (r, j) (kCell* bits; 0 outside i = -1..nx, j = -1..ny
-    // or without flags).
-    auto load_flags = [&](int r) -> unsigned int {
+    // Flag byte of cell (r, j) (kCell* bits), from a pointer that steps one row
+    // per call; columns past ny (no face of an owned cell reads them) repeat
+    // column ny's.  Called for rows i0 - 1 .. i1 in turn, all of them within the
+    // flags' -1 .. nx.
+    const uint8_t* fp = flags ? flags + static_cast<long long>(i0) * (L.ny + 2) + (min(j, L.ny) + 1) : nullptr;
+    auto load_flags = [&]() -> unsigned int {
         unsigned int f = 0u;
-        if (flags && r >= -1 && r <= L.nx) {  // uniform per warp
-            if (j <= L.ny) f = flags[static_cast<long long>(r + 1) * (L.ny + 2) + (j + 1)];
+        if (flags) {  // uniform per warp
+            f = *fp;
+            fp += L.ny + 2;
         }
         return f;
     };
@@ -924,11 +941,11 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int i0, 
             load_halo(i0, hal);
         }
     }
-    if (active_warp) f_next = load_flags(i0 - 1);
+    if (active_warp) f_next = load_flags();
     for (int r = i0 - 1; active_warp && r <= i1; ++r) {
         const unsigned int f_r = f_next;
-        f_next = load_flags(r + 1);
         if (r == i1) let_next_in();
+        else f_next = load_flags();
         if constexpr (kRing && !kU0Ring) {  // FP64 ring: U^0 of row r-1, ahead of the x reconstruction
             if (a.stage >= 1 && owner && r - 1 >= i0) ld_cell<T>(static_cast<const T*>(a.u0), L.offset(r - 1, j), pf_u0);
         }
@@ -963,7 +980,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int i0, 
         if constexpr (kPos) {
             C cc[kVars];
             full(win[2], cc);
-            fix_states<Pol>(f_r & kCellLowXhi, f_r & kCellLowXlo, cc, g, Lr, Rr);
+            fix_states_warp<Pol>(f_r, kCellLowXhi, kCellLowXlo, cc, g, Lr, Rr);
         }
         if constexpr (kL == 1) {
             if (r < i1) load_row(r + 3, nxt);
@@ -975,7 +992,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int i0, 
             // (computed on a boundary row too and replaced there: a flux in a
             // branch of its own would not overlap the surrounding work)
             hll_flux<Pol>(Lx, Rr, 0, hll, g, FX);
-            if ((r == 0 && lo_x) || (r == L.nx && hi_x)) {  // uniform per warp
+            if (kEdge && (r == wall_lo || r == wall_hi)) {  // uniform per warp
                 C c[kVars];
                 if (r == 0) full(win[2], c);
                 else full(win[1], c);
