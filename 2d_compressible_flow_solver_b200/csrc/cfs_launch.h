@@ -72,14 +72,13 @@ constexpr MarchVariant kVariants[kNumVariants] = {
 };
 // 1-based defaults, from the committed tuning table
 // (2d_compressible_flow_solver_b200/tuning.json): FP32 stages its ring rows by
-// per-lane 16-byte cp.async (variant 7: 10,937 Mcell-steps/s at 4096^2 against
-// 10,552 for the same shape staged by TMA, whose lane-0 issue and mbarrier
+// per-lane 16-byte cp.async (variant 7: 13,979 Mcell-steps/s at 4096^2 against
+// 12,871 for the same shape staged by TMA, whose lane-0 issue and mbarrier
 // waits cost more instructions than the copies they replace once cells are
-// interleaved); FP64 by cp.async too (variant 8): with the row chunk chosen per
-// launch it matches the TMA ring on periodic grids (4096^2: 5,986 against
-// 5,999; 2048^2: 5,527 against 5,523) and wins with edge code (2048^2
-// transmissive 5,186 against 5,120, with floors and a cylinder 4,734 against
-// 4,448).
+// interleaved), FP64 too (variant 8: 4096^2 7,522 against 7,089; 1024^2 5,679
+// against 5,355).  The defaults also run with the launch's scheme compiled in
+// (launch_march_default); 5 blocks of 96 registers hold the FP32 loop with edge
+// code as well.
 constexpr int kDefaultVariantF32 = 7;
 constexpr int kDefaultVariantF64 = 8;
 // FP64 ring blocks per SM (4 warps at 128 registers; 37 KB dynamic + 4.6 KB

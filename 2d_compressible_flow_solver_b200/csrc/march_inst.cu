@@ -1,6 +1,6 @@
 // Row-march launchers of one (form, feature set): compiled once per pair, with
 //   -DCFS_MARCH_POL=PolF32|PolF64  -DCFS_MARCH_FEAT=0..7  -DCFS_MARCH_FN=<launcher name>
-// (the build gives each pair its own object, so the 160 kernels compile in
+// (the build gives each pair its own object, so the kernels compile in
 // parallel).  The launcher runs the variant `v` of kVariants (1-based).
 #include <mutex>
 

@@ -62,11 +62,11 @@ WORDS_PER_CELL_STEP = 32
 MEASURED_TRAFFIC_BYTES_PER_CELL_LAUNCH = {"f32": 41.6, "f64": None}
 # Floating-point operations the FP32-mixed march executes per cell-step (its
 # three stage launches; packed FFMA2 = 4, FADD2/FMUL2/FFMA/DFMA = 2, others 1),
-# from ncu's per-opcode instruction counts (sass__inst_executed_per_opcode) of
-# the three stage launches of one step on a periodic 2048^2 run with 32-row
-# work items, as at 4096^2, and stochastic rounding in every stage (the
-# defaults).  Data-independent on smooth states.
-MEASURED_FLOPS_PER_CELL_STEP = {"f32": {"fp32": 2814.1, "fp64": 3.8}}
+# from ncu's per-opcode instruction counts of the three stage launches of one
+# step on a periodic 2048^2 run with 40-row work items, which repeat as many
+# rows as the launcher's two chunk lengths at 4096^2 do, and stochastic rounding
+# in every stage (the default).  Data-independent on smooth states.
+MEASURED_FLOPS_PER_CELL_STEP = {"f32": {"fp32": 2545.0, "fp64": 5.0}}
 # The reference's scheme as its own driver runs it (Run.cpp:41-48 with
 # TVD3rdRK, RiemmanSolverHLL, transmissive sides, fixed dt): what the
 # reference arm times, and the engine's like-for-like companion rate.

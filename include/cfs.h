@@ -131,8 +131,8 @@ typedef struct cfs_config {
     int positivity;          /* enum cfs_positivity */
     int rounding;            /* enum cfs_rounding (CFS_FP32_MIXED) */
     int march_rows;          /* throughput forms: rows of one warp's work item in the row march;
-                                0 = chosen at each launch so the blocks fill whole waves of the
-                                GPU's resident blocks (the tuned default), > 0 = fixed (<= 4096) */
+                                0 = chosen at each launch (a warp per row on small grids, else long
+                                chunks first and short ones behind them), > 0 = fixed (<= 4096) */
 } cfs_config;
 
 typedef struct cfs_ctx cfs_ctx;
@@ -353,7 +353,7 @@ int cfs_conserved_totals(cfs_ctx* ctx, double totals[4]);
 /* ---- Batched cases -------------------------------------------------------
  * Hundreds of independent grids of uneven size advanced together: every stage
  * of every case runs in ONE persistent launch whose warps pull work items
- * (case, 30-column segment, row chunk) from a device counter, largest cases first;
+ * (case, 30-column segment, rows) from a device counter, largest cases first;
  * each case keeps its own CFL time step, computed on the device; whole steps
  * are replayed from a CUDA graph.  Throughput forms only (CFS_FP32_MIXED,
  * CFS_FP64).  No reference counterpart (the reference runs one grid). */
