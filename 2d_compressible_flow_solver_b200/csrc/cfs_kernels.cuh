@@ -170,18 +170,6 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-// NaN-propagating minimum and maximum (one instruction each).
-__device__ __forceinline__ float min_nan(float a, float b) {
-    float r;
-    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float max_nan(float a, float b) {
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-
 template <class C> __device__ __forceinline__ C min_ref(C a, C b) { return (b < a) ? b : a; }
 template <class C> __device__ __forceinline__ C max_ref(C a, C b) { return (a < b) ? b : a; }
 
@@ -409,32 +397,32 @@ __device__ __forceinline__ void hll_flux(const Face5<typename Pol::C>& L, const 
         }
     }
     if constexpr (!Pol::kExact) {
-        // The HLL average written from the left flux, F = FL + w (SR dU - dF)
-        // with w = SL / (SR - SL), and the bounds clamped to SL <= 0 <= SR:
-        // where SL >= 0 the weight is 0 (F = FL exactly), where SR <= 0 it is
-        // -1 (F = FL + dF, the right flux to rounding), so no upwind selects
-        // remain.  A NaN bound stays NaN and gives a NaN flux, and the floor
-        // on SR keeps the reciprocal's argument positive.  Per face 8 packed
-        // instructions (FP32) and no selects, against 10 and 8 for the average
-        // formed from both fluxes and selected; 16 FP64 operations against 20.
+        // The HLL average written from the flux B of the side that it is nearer to,
+        //   |SL| <= |SR|:  F = FL + SL / (SR - SL) (SR dU + FL - FR),
+        //   |SR| <  |SL|:  F = FR + SR / (SR - SL) (SL dU + FL - FR),
+        // with a weight of 1/2 at most, and of 0 where the flow is supersonic (F =
+        // B exactly).  Written from the left flux throughout, a flow leaving a
+        // large state to the left formed its right flux as FL - (FL - FR): with a
+        // left state R times the right one a component was wrong by 2.2e-5 (R =
+        // 100) to 2.4e-3 (R = 1e4) of itself in FP32.  A mirrored face (Davis bounds)
+        // has the mirrored flux bit for bit, except where |SL| = |SR|.
+        const bool right = SR < -SL, up = SL >= 0 || SR <= 0;
+        const C s = right ? SL : SR;
         if constexpr (Pol::kMixed) {
-            const float SLm = min_nan(SL, 0.0f), SRp = max_nan(SR, 1e-30f);
-            const float2 w = p2(SLm * rcp_fast(SRp - SLm)), sr = p2(SRp);
+            const float2 w = p2(up ? 0.0f : (right ? SR : SL) * rcp_fast(SR - SL)), sv = p2(s);
             const float2 L01 = make_float2(FL[0], FL[1]), L23 = make_float2(FL[2], FL[3]);
-            const float2 F01 = fma2(w, fma2(sr, sub2(make_float2(R.r, R.mx), make_float2(L.r, L.mx)),
-                                            sub2(L01, make_float2(FR[0], FR[1]))), L01);
-            const float2 F23 = fma2(w, fma2(sr, sub2(make_float2(R.my, R.E), make_float2(L.my, L.E)),
-                                            sub2(L23, make_float2(FR[2], FR[3]))), L23);
+            const float2 R01 = make_float2(FR[0], FR[1]), R23 = make_float2(FR[2], FR[3]);
+            const float2 F01 = fma2(w, fma2(sv, sub2(make_float2(R.r, R.mx), make_float2(L.r, L.mx)), sub2(L01, R01)), right ? R01 : L01);
+            const float2 F23 = fma2(w, fma2(sv, sub2(make_float2(R.my, R.E), make_float2(L.my, L.E)), sub2(L23, R23)), right ? R23 : L23);
             F[0] = F01.x;
             F[1] = F01.y;
             F[2] = F23.x;
             F[3] = F23.y;
         } else {
-            const C SLm = SL >= 0 ? C(0) : SL, SRp = SR <= 0 ? C(1e-290) : SR;
-            const C w = SLm * rcp_pos(SRp - SLm);
+            const C w = up ? C(0) : (right ? SR : SL) * rcp_pos(SR - SL);
             const C dU[4] = {R.r - L.r, R.mx - L.mx, R.my - L.my, R.E - L.E};
 #pragma unroll
-            for (int q = 0; q < 4; ++q) F[q] = fma(w, fma(SRp, dU[q], FL[q] - FR[q]), FL[q]);
+            for (int q = 0; q < 4; ++q) F[q] = fma(w, fma(s, dU[q], FL[q] - FR[q]), right ? FR[q] : FL[q]);
         }
         return;
     }
