@@ -16,6 +16,17 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200, sm_100a)")
 
 
+@pytest.hookimpl(wrapper=True)
+def pytest_runtest_call(item):
+    """Tests that run the reference's own classes are skipped where those are not built."""
+    from oracle_bind import ReferenceNotBuilt
+
+    try:
+        return (yield)
+    except ReferenceNotBuilt as e:
+        pytest.skip(str(e))
+
+
 @pytest.fixture(scope="session")
 def cfsb():
     """The engine's Python binding (package folder name starts with a digit)."""

@@ -80,9 +80,17 @@ _ref = None
 _orc = None
 
 
+class ReferenceNotBuilt(OSError):
+    """The reference's classes are not built here (no reference tree); a test
+    that needs them is skipped (conftest.py)."""
+
+
 def ref_lib(perf: bool = False) -> ctypes.CDLL:
     global _ref
     ensure_built()
+    path = REF_PERF if perf else REF_STRICT
+    if not path.exists():
+        raise ReferenceNotBuilt(f"{path.name} is not built: no reference tree")
     if perf:
         lib = ctypes.CDLL(str(REF_PERF))
         lib.ref_time_stages.restype = ctypes.c_double
