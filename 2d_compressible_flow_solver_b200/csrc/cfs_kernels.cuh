@@ -400,8 +400,9 @@ __device__ __forceinline__ void hll_flux(const Face5<typename Pol::C>& L, const 
         // The HLL average written from the flux B of the side that it is nearer to,
         //   |SL| <= |SR|:  F = FL + SL / (SR - SL) (SR dU + FL - FR),
         //   |SR| <  |SL|:  F = FR + SR / (SR - SL) (SL dU + FL - FR),
-        // with a weight of 1/2 at most, and of 0 where the flow is supersonic (F =
-        // B exactly).  Written from the left flux throughout, a flow leaving a
+        // with a weight of 1/2 at most; where the flow is supersonic F = B, by a
+        // select, so that nothing downwind enters, infinite or NaN as it may be
+        // (Davis bounds drop a NaN side).  Written from the left flux throughout, a flow leaving a
         // large state to the left formed its right flux as FL - (FL - FR): with a
         // left state R times the right one a component was wrong by 2.2e-5 (R =
         // 100) to 2.4e-3 (R = 1e4) of itself in FP32.  A mirrored face (Davis bounds)
@@ -409,20 +410,33 @@ __device__ __forceinline__ void hll_flux(const Face5<typename Pol::C>& L, const 
         const bool right = SR < -SL, up = SL >= 0 || SR <= 0;
         const C s = right ? SL : SR;
         if constexpr (Pol::kMixed) {
-            const float2 w = p2(up ? 0.0f : (right ? SR : SL) * rcp_fast(SR - SL)), sv = p2(s);
+            const float2 w = p2((right ? SR : SL) * rcp_fast(SR - SL)), sv = p2(s);
             const float2 L01 = make_float2(FL[0], FL[1]), L23 = make_float2(FL[2], FL[3]);
             const float2 R01 = make_float2(FR[0], FR[1]), R23 = make_float2(FR[2], FR[3]);
-            const float2 F01 = fma2(w, fma2(sv, sub2(make_float2(R.r, R.mx), make_float2(L.r, L.mx)), sub2(L01, R01)), right ? R01 : L01);
-            const float2 F23 = fma2(w, fma2(sv, sub2(make_float2(R.my, R.E), make_float2(L.my, L.E)), sub2(L23, R23)), right ? R23 : L23);
-            F[0] = F01.x;
-            F[1] = F01.y;
-            F[2] = F23.x;
-            F[3] = F23.y;
+            const float2 X01 = fma2(sv, sub2(make_float2(R.r, R.mx), make_float2(L.r, L.mx)), sub2(L01, R01));
+            const float2 X23 = fma2(sv, sub2(make_float2(R.my, R.E), make_float2(L.my, L.E)), sub2(L23, R23));
+            float2 B01 = right ? R01 : L01, B23 = right ? R23 : L23;
+            if (!up) {
+                B01 = fma2(w, X01, B01);
+                B23 = fma2(w, X23, B23);
+            }
+            F[0] = B01.x;
+            F[1] = B01.y;
+            F[2] = B23.x;
+            F[3] = B23.y;
         } else {
-            const C w = up ? C(0) : (right ? SR : SL) * rcp_pos(SR - SL);
+            const C w = (right ? SR : SL) * rcp_pos(SR - SL);
             const C dU[4] = {R.r - L.r, R.mx - L.mx, R.my - L.my, R.E - L.E};
+            C X[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) F[q] = fma(w, fma(s, dU[q], FL[q] - FR[q]), right ? FR[q] : FL[q]);
+            for (int q = 0; q < 4; ++q) {
+                X[q] = fma(s, dU[q], FL[q] - FR[q]);
+                F[q] = right ? FR[q] : FL[q];
+            }
+            if (!up) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) F[q] = fma(w, X[q], F[q]);
+            }
         }
         return;
     }
