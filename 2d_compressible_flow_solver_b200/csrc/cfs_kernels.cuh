@@ -245,10 +245,15 @@ __device__ __forceinline__ double weno5_ref(double v0, double v1, double v2, dou
     return ok ? w : weno5_ref_divide(v0, v1, v2, v3, v4, eps);
 }
 
+// FP32: share of the square beyond its stencil that an outer indicator holds (weno5_pair_x2).
+constexpr float kWenoTiny = 1e-12f;
+
 // The same reconstruction with one division: alpha_k = d_k / q_k with
 // q_k = (eps + beta_k)^2 is scaled by q0 q1 q2, so
 // result = (sum d_k q_l q_m P_k) / (6 sum d_k q_l q_m), P_k = 6 x candidate k.
-// In FP32 beta is capped at 1e9 so that the q products stay finite.
+// In FP32, whose range those products leave at indicators of 1e9, the weights
+// are relative to the middle one (weno5_pair_x2) and normalised before they
+// multiply the candidates.
 template <class C>
 __device__ __forceinline__ C weno5_fast(C v0, C v1, C v2, C v3, C v4, C eps) {
     const C k13 = C(13.0 / 12.0), k14 = C(0.25);
@@ -258,20 +263,21 @@ __device__ __forceinline__ C weno5_fast(C v0, C v1, C v2, C v3, C v4, C eps) {
     C b0 = k13 * d0 * d0 + k14 * e0 * e0;
     C b1 = k13 * d1 * d1 + k14 * e1 * e1;
     C b2 = k13 * d2 * d2 + k14 * e2 * e2;
-    if (sizeof(C) == 4) {
-        b0 = fmin(b0, C(1e9));
-        b1 = fmin(b1, C(1e9));
-        b2 = fmin(b2, C(1e9));
-    }
-    C q0 = eps + b0, q1 = eps + b1, q2 = eps + b2;
-    q0 *= q0;
-    q1 *= q1;
-    q2 *= q2;
-    const C a0 = C(0.1) * q1 * q2, a1 = C(0.6) * q0 * q2, a2 = C(0.3) * q0 * q1;
     const C p0 = C(2) * v0 - C(7) * v1 + C(11) * v2;
     const C p1 = -v1 + C(5) * v2 + C(2) * v3;
     const C p2 = C(2) * v2 + C(5) * v3 - v4;
-    return (a0 * p0 + a1 * p1 + a2 * p2) * rcp_pos(C(6) * (a0 + a1 + a2));
+    if constexpr (sizeof(C) == 4) {
+        const C q1 = eps + b1, r0 = q1 * rcp_fast(eps + b0 + kWenoTiny * b1), r2 = q1 * rcp_fast(eps + b2 + kWenoTiny * b1);
+        const C a0 = C(0.1) * r0 * r0, a1 = C(0.6), a2 = C(0.3) * r2 * r2, i = rcp_fast(C(6) * (a0 + a1 + a2));
+        return (a0 * i) * p0 + (a1 * i) * p1 + (a2 * i) * p2;
+    } else {
+        C q0 = eps + b0, q1 = eps + b1, q2 = eps + b2;
+        q0 *= q0;
+        q1 *= q1;
+        q2 *= q2;
+        const C a0 = C(0.1) * q1 * q2, a1 = C(0.6) * q0 * q2, a2 = C(0.3) * q0 * q1;
+        return (a0 * p0 + a1 * p1 + a2 * p2) * rcp_pos(C(6) * (a0 + a1 + a2));
+    }
 }
 
 template <class Pol>
