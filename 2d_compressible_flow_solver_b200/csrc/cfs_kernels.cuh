@@ -53,8 +53,9 @@ template <class C> struct Face5 { C r, mx, my, E, p, a, ri; };
 
 // A product that is rounded by itself.  The throughput forms write every
 // multiply-add as fma() and every product that enters a sum otherwise as
-// mul(), so no contraction is left to the compiler and a cell's result is the
-// same bits in every kernel that computes it (row march, tile form, batch).
+// mul() (a product by a power of two excepted, which rounds nothing), so no
+// contraction is left to the compiler and a cell's result is the same bits in
+// every kernel that computes it (row march, tile form, batch, face fluxes).
 __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 
@@ -253,30 +254,32 @@ constexpr float kWenoTiny = 1e-12f;
 // result = (sum d_k q_l q_m P_k) / (6 sum d_k q_l q_m), P_k = 6 x candidate k.
 // In FP32, whose range those products leave at indicators of 1e9, the weights
 // are relative to the middle one (weno5_pair_x2) and normalised before they
-// multiply the candidates.
+// multiply the candidates.  (Used off the row loop, for the Dirichlet faces: in
+// FP64 the quotient is an IEEE division's.)
 template <class C>
 __device__ __forceinline__ C weno5_fast(C v0, C v1, C v2, C v3, C v4, C eps) {
     const C k13 = C(13.0 / 12.0), k14 = C(0.25);
-    const C d0 = v0 - C(2) * v1 + v2, e0 = v0 - C(4) * v1 + C(3) * v2;
-    const C d1 = v1 - C(2) * v2 + v3, e1 = v1 - v3;
-    const C d2 = v2 - C(2) * v3 + v4, e2 = C(3) * v2 - C(4) * v3 + v4;
-    C b0 = k13 * d0 * d0 + k14 * e0 * e0;
-    C b1 = k13 * d1 * d1 + k14 * e1 * e1;
-    C b2 = k13 * d2 * d2 + k14 * e2 * e2;
-    const C p0 = C(2) * v0 - C(7) * v1 + C(11) * v2;
-    const C p1 = -v1 + C(5) * v2 + C(2) * v3;
-    const C p2 = C(2) * v2 + C(5) * v3 - v4;
+    const C d0 = fma(C(-2), v1, v0) + v2, e0 = fma(C(3), v2, fma(C(-4), v1, v0));
+    const C d1 = fma(C(-2), v2, v1) + v3, e1 = v1 - v3;
+    const C d2 = fma(C(-2), v3, v2) + v4, e2 = fma(C(3), v2, fma(C(-4), v3, v4));
+    const C b0 = fma(k13 * d0, d0, mul(k14 * e0, e0));
+    const C b1 = fma(k13 * d1, d1, mul(k14 * e1, e1));
+    const C b2 = fma(k13 * d2, d2, mul(k14 * e2, e2));
+    const C p0 = fma(C(11), v2, fma(C(-7), v1, C(2) * v0));
+    const C p1 = fma(C(2), v3, fma(C(5), v2, -v1));
+    const C p2 = fma(C(5), v3, fma(C(2), v2, -v4));
     if constexpr (sizeof(C) == 4) {
-        const C q1 = eps + b1, r0 = q1 * rcp_fast(eps + b0 + kWenoTiny * b1), r2 = q1 * rcp_fast(eps + b2 + kWenoTiny * b1);
-        const C a0 = C(0.1) * r0 * r0, a1 = C(0.6), a2 = C(0.3) * r2 * r2, i = rcp_fast(C(6) * (a0 + a1 + a2));
-        return (a0 * i) * p0 + (a1 * i) * p1 + (a2 * i) * p2;
+        const C q1 = eps + b1;
+        const C r0 = mul(q1, rcp_fast(fma(kWenoTiny, b1, eps + b0))), r2 = mul(q1, rcp_fast(fma(kWenoTiny, b1, eps + b2)));
+        const C a0 = mul(C(0.1) * r0, r0), a1 = C(0.6), a2 = mul(C(0.3) * r2, r2), i = rcp_fast(C(6) * (a0 + a1 + a2));
+        return fma(mul(a0, i), p0, fma(mul(a1, i), p1, mul(mul(a2, i), p2)));
     } else {
         C q0 = eps + b0, q1 = eps + b1, q2 = eps + b2;
         q0 *= q0;
         q1 *= q1;
         q2 *= q2;
-        const C a0 = C(0.1) * q1 * q2, a1 = C(0.6) * q0 * q2, a2 = C(0.3) * q0 * q1;
-        return (a0 * p0 + a1 * p1 + a2 * p2) * rcp_pos(C(6) * (a0 + a1 + a2));
+        const C a0 = mul(C(0.1) * q1, q2), a1 = mul(C(0.6) * q0, q2), a2 = mul(C(0.3) * q0, q1);
+        return mul(fma(a0, p0, fma(a1, p1, mul(a2, p2))), rcp_fast(C(6) * (a0 + a1 + a2)));
     }
 }
 

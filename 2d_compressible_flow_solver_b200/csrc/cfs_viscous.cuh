@@ -48,7 +48,7 @@ template <> struct Pair<float> { using type = float2; };
 template <> struct Pair<double> { using type = double2; };
 __device__ __forceinline__ double2 add2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 sub2(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 mul2(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+__device__ __forceinline__ double2 mul2(double2 a, double2 b) { return make_double2(mul(a.x, b.x), mul(a.y, b.y)); }
 __device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
     return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
 }
@@ -86,13 +86,13 @@ template <class C, class V>
 __device__ __forceinline__ void visc_flux(int nrm, const ViscDir<C, V>& k, V w0, V w1, V w2, V w3, V w4, V w5, C T0, C T1,
                                           C T2, C T3, C T4, C T5, V cr, V n16, V m16, C F[3]) {
     const V dn = fma2(k.t0, sub2(w3, w2), fma2(k.t1, sub2(w4, w1), mul2(k.t2, sub2(w5, w0))));
-    const C dT = fma(k.t0.x, T3 - T2, fma(k.t1.x, T4 - T1, k.t2.x * (T5 - T0)));
+    const C dT = fma(k.t0.x, T3 - T2, fma(k.t1.x, T4 - T1, mul(k.t2.x, T5 - T0)));
     const V f = fma2(n16, add2(w2, w3), mul2(m16, add2(w1, w4)));
-    const C snn = nrm == 0 ? k.mu43 * dn.x - k.mu23 * cr.y : k.mu43 * dn.y - k.mu23 * cr.x;
-    const C snt = nrm == 0 ? k.mu * (cr.x + dn.y) : k.mu * (dn.x + cr.y);
+    const C snn = nrm == 0 ? fma(k.mu43, dn.x, -mul(k.mu23, cr.y)) : fma(k.mu43, dn.y, -mul(k.mu23, cr.x));
+    const C snt = nrm == 0 ? mul(k.mu, cr.x + dn.y) : mul(k.mu, dn.x + cr.y);
     F[0] = nrm == 0 ? snn : snt;
     F[1] = nrm == 0 ? snt : snn;
-    F[2] = fma(f.x, F[0], fma(f.y, F[1], k.kT * dT));
+    F[2] = fma(f.x, F[0], fma(f.y, F[1], mul(k.kT, dT)));
 }
 
 // Cell-centred derivatives, scaled for the interpolation that reads them:
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(32 * kViscWarps, kMinBlocks) viscous_kernel(co
         src += row_step;
         const C ri = rcp_pos(c[0]);
         uv[k] = mul2(make_pair_of(c[1], c[2]), p2(ri));
-        tt[k] = cTg * (c[3] - C(0.5) * fma(c[1], uv[k].x, c[2] * uv[k].y)) * ri;
+        tt[k] = mul(mul(cTg, fma(C(-0.5), fma(c[1], uv[k].x, mul(c[2], uv[k].y)), c[3])), ri);
         sm.uv[k][lane + 3] = uv[k];
         sm.T[k][lane + 3] = tt[k];
     };
