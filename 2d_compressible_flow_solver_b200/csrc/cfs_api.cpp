@@ -615,7 +615,7 @@ int cfs_set_state(cfs_ctx* c, const double* U) {
     c->wmax_carry = false;
     CFS_CUDA(c, cudaSetDevice(c->cfg.device));
     const size_t hb = sizeof(double) * kVars * static_cast<size_t>(c->cfg.nx) * c->cfg.ny;
-    if (c->small_state) {
+    if (c->small_state && cfs::is_host_memory(U)) {
         std::memcpy(c->small_state, U, hb);
         CFS_CUDA(c, cudaMemcpyAsync(c->staging, c->small_state, hb, cudaMemcpyHostToDevice, c->stream));
     } else {
@@ -685,10 +685,11 @@ int cfs_get_state(cfs_ctx* c, double* U) {
     CFS_CUDA(c, cudaSetDevice(c->cfg.device));
     const size_t hb = sizeof(double) * kVars * static_cast<size_t>(c->cfg.nx) * c->cfg.ny;
     // a small state is written to the pinned array by the kernel itself
-    double* const dst = c->small_state ? c->small_state : c->staging;
+    const bool small = c->small_state && cfs::is_host_memory(U);
+    double* const dst = small ? c->small_state : c->staging;
     CFS_CUDA(c, cfs::launch_unpack(c->L.elem_bytes, c->S[c->cur], dst, c->L, c->stream));
     CFS_CUDA(c, cfs::launch_results(c->results, nullptr, nullptr, c->err_d, c->stream));
-    if (c->small_state) {
+    if (small) {
         CFS_CUDA(c, cudaStreamSynchronize(c->stream));
         std::memcpy(U, c->small_state, hb);
     } else {

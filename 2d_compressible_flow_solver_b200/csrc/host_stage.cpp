@@ -99,14 +99,24 @@ int spawn(std::vector<std::thread>& pool, int n, F& work) {
 
 }  // namespace
 
-bool host_is_pageable(const void* p) {
+static bool memory_type(const void* p, cudaMemoryType& type) {
     cudaPointerAttributes at{};
-    const cudaError_t e = cudaPointerGetAttributes(&at, p);
-    if (e != cudaSuccess) {
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         (void)cudaGetLastError();  // this query's own error only
         return false;
     }
-    return at.type == cudaMemoryTypeUnregistered;
+    type = at.type;
+    return true;
+}
+
+bool host_is_pageable(const void* p) {
+    cudaMemoryType type;
+    return memory_type(p, type) && type == cudaMemoryTypeUnregistered;
+}
+
+bool is_host_memory(const void* p) {
+    cudaMemoryType type;
+    return memory_type(p, type) && (type == cudaMemoryTypeUnregistered || type == cudaMemoryTypeHost);
 }
 
 cudaError_t upload_staged(void* dst, const void* src, size_t bytes, void* stage, cudaStream_t stream, int device) {

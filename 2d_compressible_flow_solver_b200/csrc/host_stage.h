@@ -17,6 +17,10 @@ namespace cfs {
 // or managed memory): only such arrays take the staged copies.
 bool host_is_pageable(const void* p);
 
+// Whether `p` is host memory, pageable or page-locked: only such arrays are
+// copied by the host itself.
+bool is_host_memory(const void* p);
+
 // Smallest copy worth the pipeline (smaller ones go through cudaMemcpyAsync).
 constexpr size_t kStagedCopyMinBytes = size_t(32) << 20;
 
