@@ -1040,10 +1040,12 @@ int cfs_steps_stage(cfs_ctx* c, int part) {
     const int stage = c->next_stage;
     const Roles r = roles_for(c, stage, c->cur, c->u0_idx, c->u1_idx);
     // the step's first-stage bookkeeping (t, dt, CFL slot reset) runs in
-    // exactly one launch: the full stage or its interior part; the
+    // exactly one launch: the full stage or its interior part (the first edge
+    // launch where the interior has no rows, nx = 6); the
     // immersed-ghost fill and viscous RHS run with the full stage only (the
     // split parts refuse both above)
-    const bool first = stage == 0 && part != CFS_PART_EDGES;
+    const bool no_interior = c->cfg.nx == 2 * cfs::kGhost;
+    const bool first = stage == 0 && (part != CFS_PART_EDGES || no_interior);
     const bool last = stage == S - 1;
     if (part == CFS_PART_ALL) {
         const int rc = enqueue_stage(c, stage, r, 0.0, true, c->steps_parity, first, last, 0, 0, true);
@@ -1055,7 +1057,7 @@ int cfs_steps_stage(cfs_ctx* c, int part) {
     } else {
         int rc = enqueue_stage(c, stage, r, 0.0, true, c->steps_parity, first, last, 0, cfs::kGhost, false);
         if (rc == CFS_OK)
-            rc = enqueue_stage(c, stage, r, 0.0, true, c->steps_parity, first, last, c->cfg.nx - cfs::kGhost,
+            rc = enqueue_stage(c, stage, r, 0.0, true, c->steps_parity, false, last, c->cfg.nx - cfs::kGhost,
                                c->cfg.nx, false);
         if (rc != CFS_OK) return rc;
     }
