@@ -68,8 +68,12 @@ struct cfs_ctx {
     double* totals = nullptr;
     cudaGraphExec_t graph2 = nullptr;  // two full steps (parity 0 then 1)
     cudaGraphExec_t graph1 = nullptr;  // one full step (parity 0): an odd step count's last step
-    cfs::HostResults* results = nullptr;  // pinned; behind it, for a small grid, its host-order state (small_state)
-    double* small_state = nullptr;        // null: states move by copies
+    // What the host reads back: written by the device in pinned memory (results
+    // and results_dev the same), or, where that is refused, in device memory and copied.
+    cfs::HostResults* results = nullptr;
+    cfs::HostResults* results_dev = nullptr;
+    cfs::HostResults results_copy{};
+    double* small_state = nullptr;  // behind pinned results, for a small grid: its host-order state; null: states move by copies
     // device-ordered stepping (cfs_steps_*): between begin and end
     bool in_steps = false;
     bool steps_cfl = false;
@@ -220,11 +224,20 @@ int report_device_errors(cfs_ctx* c, unsigned int e) {
     return CFS_OK;
 }
 
+// Waits for the stream; c->results then holds what the device wrote.
+cudaError_t wait_stream(cfs_ctx* c) {
+    if (c->results_dev != c->results) {
+        const cudaError_t e = cudaMemcpyAsync(c->results, c->results_dev, sizeof(cfs::HostResults), cudaMemcpyDeviceToHost, c->stream);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaStreamSynchronize(c->stream);
+}
+
 // Waits for the stream and reads back its results: the step parameters (when
 // asked for) and the error flags.
 int wait_results(cfs_ctx* c, cfs::DevParams* params) {
-    CFS_CUDA(c, cfs::launch_results(c->results, params ? c->P : nullptr, nullptr, c->err_d, c->stream));
-    CFS_CUDA(c, cudaStreamSynchronize(c->stream));
+    CFS_CUDA(c, cfs::launch_results(c->results_dev, params ? c->P : nullptr, nullptr, c->err_d, c->stream));
+    CFS_CUDA(c, wait_stream(c));
     if (params) *params = c->results->params;
     return report_device_errors(c, c->results->err);
 }
@@ -520,12 +533,17 @@ int cfs_create(const cfs_config* cfg, cfs_ctx** out) {
     cudaMemsetAsync(c->wmax, 0, sizeof(unsigned long long), c->stream);
     const size_t small = hb <= kSmallStateBytes ? hb : 0;
     void* pinned = nullptr;
-    if (cudaHostAlloc(&pinned, sizeof(cfs::HostResults) + small, cudaHostAllocDefault) != cudaSuccess) {
-        c->err = "pinned host allocation of the results failed";
-        return bail(CFS_ERR_NOMEM);
+    if (cudaHostAlloc(&pinned, sizeof(cfs::HostResults) + small, cudaHostAllocDefault) == cudaSuccess) {
+        c->results = c->results_dev = static_cast<cfs::HostResults*>(pinned);
+        if (small) c->small_state = reinterpret_cast<double*>(c->results + 1);
+    } else {
+        (void)cudaGetLastError();
+        c->results = &c->results_copy;
+        if (cudaMalloc(&c->results_dev, sizeof(cfs::HostResults)) != cudaSuccess) {
+            c->err = "device allocation of the results failed";
+            return bail(CFS_ERR_NOMEM);
+        }
     }
-    c->results = static_cast<cfs::HostResults*>(pinned);
-    if (small) c->small_state = reinterpret_cast<double*>(c->results + 1);
     if (c->prec != cfs::kF64Exact) {
         // tensor maps of the three state buffers (TMA load schedule), encoded
         // on the host once (the buffers never move) and passed in each
@@ -568,7 +586,8 @@ int cfs_destroy(cfs_ctx* c) {
     cudaFree(c->ib_img);
     cudaFree(c->ib_fac);
     cudaFree(c->P);
-    if (c->results) cudaFreeHost(c->results);
+    if (c->results_dev == c->results) cudaFreeHost(c->results_dev);
+    else cudaFree(c->results_dev);
     cudaFree(c->wmax);
     cudaFree(c->totals);
     cudaFree(c->err_d);
@@ -627,8 +646,8 @@ int cfs_set_state(cfs_ctx* c, const double* U) {
         const size_t n = static_cast<size_t>(c->cfg.nx) * c->cfg.ny;
         double sums[kVars] = {0, 0, 0, 0};
         if (!c->fixed_offsets) {
-            CFS_CUDA(c, cfs::launch_plane_sums(c->staging, static_cast<long long>(n), c->sums, c->results->sums, c->stream));
-            CFS_CUDA(c, cudaStreamSynchronize(c->stream));
+            CFS_CUDA(c, cfs::launch_plane_sums(c->staging, static_cast<long long>(n), c->sums, c->results_dev->sums, c->stream));
+            CFS_CUDA(c, wait_stream(c));
             std::memcpy(sums, c->results->sums, sizeof(sums));
         }
         bool changed = false;
@@ -688,13 +707,10 @@ int cfs_get_state(cfs_ctx* c, double* U) {
     const bool small = c->small_state && cfs::is_host_memory(U);
     double* const dst = small ? c->small_state : c->staging;
     CFS_CUDA(c, cfs::launch_unpack(c->L.elem_bytes, c->S[c->cur], dst, c->L, c->stream));
-    CFS_CUDA(c, cfs::launch_results(c->results, nullptr, nullptr, c->err_d, c->stream));
-    if (small) {
-        CFS_CUDA(c, cudaStreamSynchronize(c->stream));
-        std::memcpy(U, c->small_state, hb);
-    } else {
-        CFS_CUDA(c, copy_out(c, U, c->staging, hb));
-    }
+    CFS_CUDA(c, cfs::launch_results(c->results_dev, nullptr, nullptr, c->err_d, c->stream));
+    if (!small) CFS_CUDA(c, copy_out(c, U, c->staging, hb));
+    if (small || c->results_dev != c->results) CFS_CUDA(c, wait_stream(c));  // (copy_out has waited)
+    if (small) std::memcpy(U, c->small_state, hb);
     return report_device_errors(c, c->results->err);
 }
 
@@ -882,8 +898,8 @@ int cfs_compute_dt(cfs_ctx* c, double cfl, double* dt) {
     CFS_CUDA(c, cudaSetDevice(c->cfg.device));
     CFS_CUDA(c, cfs::launch_wmax(c->L.elem_bytes, c->S[c->cur], c->L, c->has_types ? c->types_d : nullptr, c->cfg.gamma,
                                  c->dx, c->dy, c->wmax, c->stream));
-    CFS_CUDA(c, cfs::launch_results(c->results, nullptr, c->wmax, nullptr, c->stream));
-    CFS_CUDA(c, cudaStreamSynchronize(c->stream));
+    CFS_CUDA(c, cfs::launch_results(c->results_dev, nullptr, c->wmax, nullptr, c->stream));
+    CFS_CUDA(c, wait_stream(c));
     double m;
     std::memcpy(&m, &c->results->wmax, sizeof(m));
     if (!(m > 0) || !std::isfinite(m))

@@ -78,7 +78,7 @@ struct DevParams {
 };
 
 // What the host reads back after a wait, in pinned memory that the device
-// writes directly.
+// writes directly (where pinned memory is refused: device memory, copied).
 struct HostResults {
     DevParams params;             // cfs_advance
     double sums[4];               // plane sums of an uploaded state
