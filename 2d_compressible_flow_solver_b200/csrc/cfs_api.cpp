@@ -35,7 +35,7 @@ struct cfs_ctx {
     double* sums = nullptr;  // plane sums of an uploaded state (FP32 storage offsets)
     void* host_stage = nullptr;   // pinned host buffer of the staged copies of large pageable arrays
     size_t host_stage_bytes = 0;
-    void* rv = nullptr;   // viscous RHS [nx][ny][4] (Navier-Stokes form only)
+    void* rv = nullptr;   // viscous RHS [nx][ny][3] (Navier-Stokes form only)
     uint8_t* types_d = nullptr;
     uint8_t* lowo_d = nullptr;  // [nx+1][ny+1] face flags of CFS_POSITIVITY_BODY
     uint8_t* cflags_d = nullptr;  // [nx+2][ny+2] per-cell flags of the row march (with cell types)
@@ -511,7 +511,7 @@ int cfs_create(const cfs_config* cfg, cfs_ctx** out) {
         return bail(CFS_ERR_NOMEM);
     }
     if (cfg->viscous == CFS_VISCOUS_NS) {
-        const size_t vb = static_cast<size_t>(kVars) * cfg->nx * cfg->ny * c->L.elem_bytes;
+        const size_t vb = static_cast<size_t>(cfs::kRvWords) * cfg->nx * cfg->ny * c->L.elem_bytes;
         if (cudaMalloc(&c->rv, vb) != cudaSuccess) { c->err = "device allocation of the viscous RHS failed"; return bail(CFS_ERR_NOMEM); }
         cudaMemsetAsync(c->rv, 0, vb, c->stream);
     }

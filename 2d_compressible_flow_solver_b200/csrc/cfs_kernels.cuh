@@ -143,6 +143,14 @@ __device__ __forceinline__ void st_cell(T* U, long long cell, const T v[kVars]) 
     }
 }
 
+// A cell's viscous RHS (kRvWords words, so scalar accesses: a warp's are
+// consecutive).
+template <class T>
+__device__ __forceinline__ void ld_rv(const T* rv, long long cell, T v[kRvWords]) {
+#pragma unroll
+    for (int q = 0; q < kRvWords; ++q) v[q] = rv[cell * kRvWords + q];
+}
+
 // State storage: FP64 holds the value; FP32 holds value - L.off[v].
 template <class T>
 __device__ __forceinline__ double dec(T stored, const Layout& L, int v) {
@@ -757,7 +765,7 @@ __global__ void __launch_bounds__((TI + 1) * TJ, kMinBlocks) stage_kernel(const 
                 rv = -double(sFX[v][ti + 1][tj] - sFX[v][ti][tj]) / a.dx - double(sFY[v][ti][tj + 1] - sFY[v][ti][tj]) / a.dy;
             }
             if (a.rv && v >= 1)
-                rv += double(static_cast<const T*>(a.rv)[Layout::at(static_cast<long long>(i) * L.ny + j, v - 1)]);
+                rv += double(static_cast<const T*>(a.rv)[(static_cast<long long>(i) * L.ny + j) * kRvWords + v - 1]);
             const double cur = double(sU[v][ti + kGhost][tj + kGhost]);
             double val = cur;
             if (fluid) {

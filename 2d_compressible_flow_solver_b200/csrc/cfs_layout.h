@@ -104,7 +104,7 @@ struct StageArgs {
     int parity;            // graph mode: which wmax slot holds this step's max
     int last_stage;        // 1: accumulate the CFL max of the new state into P->wmax[1-parity]
     int first_stage;       // 1: reset P->wmax[1-parity], advance P->t
-    const void* rv;        // optional viscous RHS (rho u, rho v, E, unused) [nx][ny][4], storage type
+    const void* rv;        // optional viscous RHS (rho u, rho v, E) [nx][ny][3], storage type
     int variant;           // throughput-form kernel variant (1-based; 0 = default)
     int positivity;        // 0 off, 1 face-state fallback, 2 also first order near the body, 3 also floors
     const uint8_t* lowo;   // positivity 2: [nx+1][ny+1] face flags, bit 0 x-face (i-1/2, j),
@@ -195,8 +195,10 @@ CFS_HD int march_features(const StageArgs& a) {
     return (a.positivity ? kFeatPos : 0) | ((a.rhs || a.rv) ? kFeatExtra : 0) | (edge ? kFeatEdge : 0);
 }
 
+constexpr int kRvWords = 3;  // words of a cell's viscous RHS
+
 // Viscous (Navier-Stokes) RHS of one state: (dFv/dx + dGv/dy) for the momentum
-// and energy equations, written to rv[nx][ny][4] (the fourth word 0).
+// and energy equations, written to rv[nx][ny][3].
 struct ViscArgs {
     const void* in;
     void* rv;

@@ -546,7 +546,7 @@ __device__ __forceinline__ void begin_step(const StageArgs& a, double dt) {
 template <class Pol, int kFeat>
 __device__ __forceinline__ void update_cell(const StageArgs& a, const UpdateCoefs& k, int i, int j,
                                             const typename Pol::C FX[kVars], const typename Pol::C FXp[kVars],
-                                            const typename Pol::C RY[kVars], const typename Pol::T rvc[kVars],
+                                            const typename Pol::C RY[kVars], const typename Pol::T rvc[kRvWords],
                                             const typename Pol::T cur[kVars], const typename Pol::T u0[kVars],
                                             const typename Pol::T u1[kVars], bool fluid, double& wloc) {
     using T = typename Pol::T;
@@ -929,7 +929,7 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int i0, 
     C FXp[kVars] = {C(0), C(0), C(0), C(0)};   // x-flux through the lower face of the previous row
     C RY[kVars] = {C(0), C(0), C(0), C(0)};    // y part of the previous row's RHS
     unsigned int f_prev = 0u, f_next = 0u;     // flags of rows r-1 and r+1
-    T rv_cur[kVars] = {T(0), T(0), T(0), T(0)}, rv_pf[kVars] = {T(0), T(0), T(0), T(0)};  // kExtra: viscous RHS of rows r-1, r
+    T rv_cur[kRvWords] = {T(0), T(0), T(0)}, rv_pf[kRvWords] = {T(0), T(0), T(0)};  // kExtra: viscous RHS of rows r-1, r
     double wloc = 0.0;
     if (active_warp && kRing) {
         if constexpr (kTma) __syncwarp();  // a previous item's reads of the ring end before lane 0's copies
@@ -955,8 +955,8 @@ __device__ __forceinline__ bool march_item(const StageArgs& a, int seg, int i0, 
         }
         if constexpr (kExtra) {  // viscous RHS of row r, a whole iteration ahead of its update
 #pragma unroll
-            for (int q = 0; q < 3; ++q) rv_cur[q] = rv_pf[q];
-            if (rv_in && owner && r >= i0 && r < i1) ld_cell<T>(rv_in, static_cast<long long>(r) * L.ny + j, rv_pf);
+            for (int q = 0; q < kRvWords; ++q) rv_cur[q] = rv_pf[q];
+            if (rv_in && owner && r >= i0 && r < i1) ld_rv<T>(rv_in, static_cast<long long>(r) * L.ny + j, rv_pf);
         }
         if constexpr (kRing) {
             // every lane is done with the previous iteration's slots; the slot

@@ -70,7 +70,8 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) tile_kernel(const __g
     // row (columns past the padded row repeat its last one: their lanes feed no owner)
     const int jmax = L.ny + kGhost - 1;
     C win[5][kVars], st[5][kVars];
-    T u0c[kVars] = {T(0), T(0), T(0), T(0)}, u1c[kVars] = {T(0), T(0), T(0), T(0)}, rvc[kVars] = {T(0), T(0), T(0), T(0)};
+    T u0c[kVars] = {T(0), T(0), T(0), T(0)}, u1c[kVars] = {T(0), T(0), T(0), T(0)};
+    T rvc[kRvWords] = {T(0), T(0), T(0)};
     unsigned int f_r = 0u;
     if (active) {
 #pragma unroll
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) tile_kernel(const __g
     if (owner) {
         if (a.stage >= 1) ld_cell<T>(static_cast<const T*>(a.u0), L.offset(r, j), u0c);
         if (uc.x1_u1) ld_cell<T>(static_cast<const T*>(a.u1), L.offset(r, j), u1c);
-        if (kExtra && a.rv) ld_cell<T>(static_cast<const T*>(a.rv), static_cast<long long>(r) * L.ny + j, rvc);
+        if (kExtra && a.rv) ld_rv<T>(static_cast<const T*>(a.rv), static_cast<long long>(r) * L.ny + j, rvc);
     }
     // ---- x reconstruction of row r; its left state to the row above
     Face5<C> Lr{}, Rr{};

@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(32 * kViscWarps, kMinBlocks) viscous_kernel(co
         if (k >= 1) y_derivative(k);  // (row i0-3's is not read)
     }
     x_face(W - 1, FXp);
-    T* out = static_cast<T*>(a.rv) + (static_cast<long long>(i0) * L.ny + j) * kVars;
+    T* out = static_cast<T*>(a.rv) + (static_cast<long long>(i0) * L.ny + j) * kRvWords;
     for (int pb = i0; pb < i1; pb += W) {
 #pragma unroll
         for (int k = 0; k < W; ++k) {
@@ -191,16 +191,14 @@ __global__ void __launch_bounds__(32 * kViscWarps, kMinBlocks) viscous_kernel(co
             const C* t = &sm.T[(k + 3) % W][lane + 1];
             visc_flux<C, V>(1, Y, w[0], w[1], w[2], w[3], w[4], w[5], t[0], t[1], t[2], t[3], t[4], t[5],
                             cross_of(gx[lane], gx[lane + 1], gx[lane + 2], gx[lane + 3], minus9), n16, m16, GY);
-            T o[kVars];
 #pragma unroll
-            for (int v = 0; v < 3; ++v) {
+            for (int v = 0; v < kRvWords; ++v) {
                 const C below = __shfl_up_sync(0xffffffffu, GY[v], 1);
-                o[v] = T((FX[v] - FXp[v]) + (GY[v] - below));
+                const T o = T((FX[v] - FXp[v]) + (GY[v] - below));
+                if (stores) out[v] = o;
                 FXp[v] = FX[v];
             }
-            o[3] = T(0);
-            if (stores) st_cell<T>(out, 0, o);
-            out += static_cast<long long>(L.ny) * kVars;
+            out += static_cast<long long>(L.ny) * kRvWords;
         }
     }
 }
