@@ -496,16 +496,14 @@ class Batch:
     """Many independent grids advanced together (a ``cfs_batch``): one
     persistent launch per stage for all cases, per-case CFL dt on the device.
     A case without ``rows`` has its work units cut by the library, with the
-    work that the stage has left (``cfs_case.rows`` = 0).  ``tuned_rows`` is
-    accepted and changes nothing: the rows of ``tuning.json`` (``batch_rows``)
-    were taken from it while units had one length per case; against the
-    library's units they lose in every batch measured (256 cases of 64..768
-    cells, FP32 3,902 against 3,745 us a step; 512 cases 7,800 against 7,629;
-    FP64 7,558 against 7,252 and 15,123 against 14,820)."""
+    work that the stage has left, and as many rows long at most as the autotuner
+    measured best for the case's size (``tuning.json`` ``batch_rows``;
+    ``tuned_rows=False``: the library's 96)."""
 
     def __init__(self, cases, *, precision: int = FP32_MIXED, rk: int = RK_SSP3, hll: int = HLL_DAVIS,
                  gamma: float = 1.4, weno_eps: float = 1e-2, device: int = 0, positivity: int = POSITIVITY_OFF,
                  rounding: int = ROUND_STOCHASTIC_ALL, tuned_rows: bool = True):
+        from . import autotune as _autotune
         self._lib = load_library()
         cfg = CfsConfig()
         self._lib.cfs_config_default(ctypes.byref(cfg))
@@ -529,6 +527,8 @@ class Batch:
                 d.npoints = int(c.get("npoints", 400))
                 d.ib_mode = int(c.get("ib_mode", IB_BILINEAR_SLIP))
             d.rows = int(c.get("rows", 0))
+            if d.rows == 0 and tuned_rows:
+                d.rows = -_autotune.batch_rows_for("f32" if precision == FP32_MIXED else "f64", d.nx, d.ny)
             d.edge_code = int(bool(c.get("edge_code", False)))
             self.shapes.append((d.nx, d.ny))
         self._b = ctypes.c_void_p()

@@ -8,15 +8,15 @@ the engine's stream, and writes the table to ``tuning.json`` next to this file:
 ``best_variant(precision, cells)`` reads it back for callers that create
 solvers (the benchmark, the batched runner).
 
-For the batched engine it also tunes the rows of a work unit (one warp's
-segment of a case, marched over that many rows) per case-size bucket, on the
-uneven batch itself: a pass of coordinate descent over the buckets, each
-trying the candidate rows with the others fixed, writing
+For the batched engine it also tunes how many rows a work unit (one warp's
+segment of a case, marched over those rows) may have at most, per case-size
+bucket, on the uneven batch itself: a pass of coordinate descent over the
+buckets, each trying the candidates with the others fixed, writing
 ``batch_rows[precision] = {"rows": {bucket: rows}, ...}`` beside the variant
-table.  (Uniform batches of one size prefer shorter units than the same sizes
-among larger cases do, so the sweep runs on the mixed workload.)
-``batch_rows_for(precision, nx, ny)`` reads it back, for a caller that fixes
-``rows`` per case; units that the library cuts itself (``rows`` = 0) are faster.
+table.  (The library cuts the units by the work that a stage has left; the
+limit is what the long ones, which run first, are cut to.)
+``batch_rows_for(precision, nx, ny)`` reads it back: the Batch wrapper limits
+every case whose rows are not set to the rows of its bucket.
 
 Usage (on a GPU): ``python -m 2d_compressible_flow_solver_b200.autotune`` is not
 importable by name, so run ``python 2d_compressible_flow_solver_b200/autotune.py
@@ -101,12 +101,12 @@ def _bucket(nx: int, ny: int) -> int:
 def time_batch(cfsb, wl, prec: int, rows_of: dict, ncases: int = 512, steps: int = 12) -> float:
     """Mcell-steps/s of the uneven batch (`ncases` cases, nx, ny in 64..768,
     half four-quadrant, half Mach 2-3 cylinder) whose cases of each size
-    bucket march work units of rows_of[bucket] rows, timed with CUDA events on
-    the batch's stream."""
+    bucket march work units of rows_of[bucket] rows at most, timed with CUDA
+    events on the batch's stream."""
     import torch
 
     cases, states = wl.batch_cases(ncases, seed=1)
-    cases = [dict(c, rows=rows_of[_bucket(c["nx"], c["ny"])]) for c in cases]
+    cases = [dict(c, rows=-rows_of[_bucket(c["nx"], c["ny"])]) for c in cases]
     with cfsb.Batch(cases, precision=prec, positivity=cfsb.POSITIVITY_FLOOR, tuned_rows=False) as b:
         cells, _ = b.info()
         for k, U in enumerate(states):
@@ -122,8 +122,8 @@ def time_batch(cfsb, wl, prec: int, rows_of: dict, ncases: int = 512, steps: int
         return cells * steps / (e0.elapsed_time(e1) / 1e3) / 1e6
 
 
-def tune_batch(precisions, doc: dict, candidates=(16, 32, 64, 96), start: int = 64) -> dict:
-    """Adds doc["batch_rows"]: work-unit rows per precision and case-size
+def tune_batch(precisions, doc: dict, candidates=(24, 48, 96, 192), start: int = 96) -> dict:
+    """Adds doc["batch_rows"]: the longest work unit per precision and case-size
     bucket, by one pass of coordinate descent on the uneven batch itself (the
     rows that suit a bucket depend on the cases beside it: units run largest
     case first, so the small cases fill the launch's tail)."""
@@ -155,7 +155,7 @@ def tune_batch(precisions, doc: dict, candidates=(16, 32, 64, 96), start: int = 
 
 
 def batch_rows_for(precision: str, nx: int, ny: int, table_path: Path = TABLE) -> int:
-    """Tuned work-unit rows for a batch case of nx x ny cells (its size
+    """Tuned longest work unit (rows) for a batch case of nx x ny cells (its size
     bucket); 0 (the library default) without a table."""
     try:
         rows = json.loads(table_path.read_text())["batch_rows"][precision]["rows"]
@@ -191,7 +191,7 @@ def main():
     ap.add_argument("--sizes", default="128,256,512,1024,2048,4096")
     ap.add_argument("--precisions", default="f32,f64")
     ap.add_argument("--out", default=str(TABLE))
-    ap.add_argument("--batch", type=int, default=1, help="1: also tune the batch work-unit rows per case size")
+    ap.add_argument("--batch", type=int, default=1, help="1: also tune the longest batch work unit per case size")
     a = ap.parse_args()
     out = Path(a.out)
     doc = tune([int(x) for x in a.sizes.split(",")], a.precisions.split(","), out)

@@ -117,8 +117,8 @@ constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
 
 // Work units of one launch: the cases order[0 .. n), the largest first.  The
 // rows of a case that sets none are cut with the work that is left: a unit gets
-// 0.7 of what remains for each of the `warps` resident ones (96 rows at most),
-// down to 0.8 sqrt(rows per warp).  Long units first repeat few rows (each
+// 0.7 of what remains for each of the `warps` resident ones (96 rows at most, or
+// -rows where that is negative), down to 0.8 sqrt(rows per warp).  Long units first repeat few rows (each
 // repeats 2), and the warps, which draw their units from one counter, end
 // together on the short ones.  Against equal units of the length that balances
 // the two (16 to 30 rows on these batches), SSP3 steps FP32 / FP64: 4 cases to
@@ -140,11 +140,12 @@ void append_units(const std::vector<BatchCase>& cases, const int* order, int n, 
     for (int k = 0; k < n; ++k) {
         const int ci = order[k];
         const BatchCase& c = cases[ci];
+        const int longest = c.desc.rows < 0 ? -std::max(c.desc.rows, -c.desc.nx) : cfs::kBatchMaxRows;
         for (int i0 = 0; i0 < c.desc.nx;) {
             int rows = c.desc.rows;
             if (rows <= 0) {
-                const double share = std::min(0.7 * left / static_cast<double>(warps), double(cfs::kBatchMaxRows));
-                rows = std::max(r_min, static_cast<int>(share + 0.5));
+                const double share = std::min(0.7 * left / static_cast<double>(warps), double(longest));
+                rows = std::min(longest, std::max(r_min, static_cast<int>(share + 0.5)));
                 left -= static_cast<double>(c.nseg) * std::min(rows, c.desc.nx - i0);
             }
             const int i1 = i0 + std::min(rows, c.desc.nx - i0);

@@ -366,8 +366,8 @@ typedef struct cfs_case {
     double radius, cx, cy;
     int npoints;
     int ib_mode;             /* enum cfs_ib_mode */
-    int rows;                /* row chunk of a work item (0: cut by the work the launch has left, from 96 rows at
-                                most down to a few) */
+    int rows;                /* rows of a work item: 0: cut by the work the launch has left, from 96 rows at most
+                                down to a few; < 0: the same, -rows at most; > 0: fixed */
     int edge_code;           /* 1: run this case with the row march's edge code even where it
                                 needs none (no physical side, no body): its work items join the
                                 launch of the cases that need it, one launch fewer per stage when
