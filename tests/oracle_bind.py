@@ -9,6 +9,7 @@ Both take and return conserved states as float64 arrays of shape (4, nx, ny).
 from __future__ import annotations
 
 import ctypes
+import errno
 import subprocess
 from pathlib import Path
 
@@ -80,17 +81,14 @@ _ref = None
 _orc = None
 
 
-class ReferenceNotBuilt(OSError):
-    """The reference's classes are not built here (no reference tree); a test
-    that needs them is skipped (conftest.py)."""
-
-
 def ref_lib(perf: bool = False) -> ctypes.CDLL:
     global _ref
     ensure_built()
     path = REF_PERF if perf else REF_STRICT
     if not path.exists():
-        raise ReferenceNotBuilt(f"{path.name} is not built: no reference tree")
+        # (a builtin exception: it also travels from worker processes to parents
+        # that cannot import this module; conftest.py skips the tests that meet it)
+        raise FileNotFoundError(errno.ENOENT, "not built, no reference tree", str(path))
     if perf:
         lib = ctypes.CDLL(str(REF_PERF))
         lib.ref_time_stages.restype = ctypes.c_double
