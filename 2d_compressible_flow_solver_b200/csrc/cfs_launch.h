@@ -72,11 +72,11 @@ constexpr MarchVariant kVariants[kNumVariants] = {
 };
 // 1-based defaults, from the committed tuning table
 // (2d_compressible_flow_solver_b200/tuning.json): FP32 stages its ring rows by
-// per-lane 16-byte cp.async (variant 7: 13,979 Mcell-steps/s at 4096^2 against
-// 12,871 for the same shape staged by TMA, whose lane-0 issue and mbarrier
+// per-lane 16-byte cp.async (variant 7: 13,997 Mcell-steps/s at 4096^2 against
+// 12,717 for the same shape staged by TMA, whose lane-0 issue and mbarrier
 // waits cost more instructions than the copies they replace once cells are
-// interleaved), FP64 too (variant 8: 4096^2 7,522 against 7,089; 1024^2 5,679
-// against 5,355).  The defaults also run with the launch's scheme compiled in
+// interleaved), FP64 too (variant 8: 4096^2 7,302 against 6,984; 1024^2 5,550
+// against 5,302).  The defaults also run with the launch's scheme compiled in
 // (launch_march_default); 5 blocks of 96 registers hold the FP32 loop with edge
 // code as well.
 constexpr int kDefaultVariantF32 = 7;

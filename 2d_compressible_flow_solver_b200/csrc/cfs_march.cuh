@@ -375,7 +375,7 @@ __device__ __forceinline__ void fix_states(bool lowL, bool lowR, const typename 
 // which lowL and lowR mark the low-order faces.  One test over both states and
 // a branch that the warp takes as one (tested and branched per lane, with the
 // flags' address and range test formed in every row, the kernel of a cylinder
-// grid ran 830 instructions per cell-stage in FP32, now 787; 48 batched cases
+// grid ran 830 instructions per cell-stage in FP32, 787 with it; 48 batched cases
 // 846 -> 818 us a step).
 template <class Pol>
 __device__ __forceinline__ void fix_states_warp(unsigned int f, unsigned int lowL, unsigned int lowR,

@@ -23,15 +23,17 @@
 // have all their values, and row q-3 is finished.  u and v of a lane share
 // packed FP32 instructions.
 //
-// Bound by instruction issue (200 instructions per cell in FP32, 0.61 issued a
+// Bound by instruction issue (202 instructions per cell in FP32, 0.61 issued a
 // cycle) and, cold, by its loads.  The kernel before worked on 16 x 32 tiles
 // (FP64 8 x 32) with a 3-cell halo, five phases through shared memory with
 // block barriers between them: 526 instructions per cell.  2048^2 FP32: 87 ->
 // 45 us a launch (ncu, cold); whole Navier-Stokes SSP3 steps 1024^2 FP32 177
-// -> 155 us, 2048^2 FP64 1,091 (an earlier form of this kernel) -> 928.
+// -> 155 us, 2048^2 FP64 1,091 (an earlier form of this kernel) -> 928.  Three
+// words a cell stored, in scalar stores: 1024^2 145.5 us with a fourth, unused
+// word in one 16-byte store, 144.2 without.
 // 26 columns a warp rather than 28 with a second pass for two halo columns:
 // the pass would cost more than the two lanes.  5 blocks of 4 warps per SM in
-// FP32 (92 registers) and 3 in FP64 (158): 4 blocks of either ran 2048^2 3 to
+// FP32 (89 registers) and 3 in FP64 (158): 4 blocks of either ran 2048^2 3 to
 // 4 % slower, FP64 with spills.
 #pragma once
 #include "cfs_kernels.cuh"
