@@ -25,6 +25,7 @@ importable by name, so run ``python 2d_compressible_flow_solver_b200/autotune.py
 from __future__ import annotations
 
 import argparse
+import functools
 import importlib
 import json
 import sys
@@ -154,11 +155,17 @@ def tune_batch(precisions, doc: dict, candidates=(24, 48, 96, 192), start: int =
     return doc
 
 
+@functools.lru_cache(maxsize=4)
+def _table(path: Path, mtime_ns: int) -> dict:
+    """The table at `path` as of `mtime_ns` (a batch asks once per case)."""
+    return json.loads(path.read_text())
+
+
 def batch_rows_for(precision: str, nx: int, ny: int, table_path: Path = TABLE) -> int:
     """Tuned longest work unit (rows) for a batch case of nx x ny cells (its size
     bucket); 0 (the library default) without a table."""
     try:
-        rows = json.loads(table_path.read_text())["batch_rows"][precision]["rows"]
+        rows = _table(table_path, table_path.stat().st_mtime_ns)["batch_rows"][precision]["rows"]
     except (OSError, KeyError, ValueError, TypeError):
         return 0
     return int(rows.get(str(_bucket(nx, ny)), 0))
